@@ -24,11 +24,13 @@ struct MoveSmem {
   double delrc, rande;
   double r[7], dis_delr, dis_rot;  // the trial's random numbers and step sizes (select_move)
   double ewld1, ewld2, vdw, ewld3, estep;
-  double x[2 * kBatchMaxSites], y[2 * kBatchMaxSites], z[2 * kBatchMaxSites], q[2 * kBatchMaxSites];
+  // trial sites (old ones first): position, charge factor q r4pie0 (negative for the old sites of a
+  // displacement, whose energies are subtracted) and atom type
+  double x[2 * kBatchMaxSites], y[2 * kBatchMaxSites], z[2 * kBatchMaxSites], cq[2 * kBatchMaxSites];
   int type[2 * kBatchMaxSites];
-  // real-space work list: per trial site its voxel-list start/length and the prefix of
-  // candidates (voxel entries + every guest site) over the sites
-  int vb[2 * kBatchMaxSites], vl[2 * kBatchMaxSites], pre[2 * kBatchMaxSites + 1];
+  // real-space work list: per trial site its voxel-list start/length and the prefix over the sites
+  // of its chunks of 32 candidates (voxel entries, then every guest site)
+  int vb[2 * kBatchMaxSites], vl[2 * kBatchMaxSites], cpre[2 * kBatchMaxSites + 1];
   int gpre[kMaxGuestTypes + 1];
   double lrc_term[kBatchMaxTab];
   // multi-jump (gcmc.f:1557-1785) across the two loop trips of one move: stage 1 while the
@@ -39,6 +41,44 @@ struct MoveSmem {
   double mj_estep, mj_energy0;
   double mj_old[3 * kBatchMaxSites];
 };
+
+// A CTA's shared memory: the chain's control block, the move in progress and the system's constants,
+// then the arrays sized by the batch (BatchArrays).  Every device function reaches it through
+// batch_smem() instead of taking references, so that its accesses compile to shared-memory
+// instructions also where the function is not inlined (a reference is a generic address there).
+struct BatchSmem {
+  ChainDev C;
+  MoveSmem M;
+  SysConst Y;
+  double red[3 * 16];  // per warp {sum akk d|S|^2, ewld2, vdw}
+  int prow[(kBatchMaxTypes + 1) * (kBatchMaxTypes + 1)];
+};
+
+__device__ __forceinline__ BatchSmem& batch_smem() {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  return *reinterpret_cast<BatchSmem*>(smem_raw);
+}
+
+constexpr int kBatchSmemBytes = ((int)sizeof(BatchSmem) + 15) & ~15;
+
+// S(k), S_new, akk, the packed k-vectors and the trial's phase tables.
+struct BatchArrays {
+  double2 *Sk, *Sn;
+  double* ak;
+  int* kp;
+  double2* tab;
+};
+
+__device__ __forceinline__ BatchArrays batch_arrays(int kmax_smem) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  BatchArrays A;
+  A.Sk = reinterpret_cast<double2*>(smem_raw + kBatchSmemBytes);
+  A.Sn = A.Sk + kmax_smem;
+  A.ak = reinterpret_cast<double*>(A.Sn + kmax_smem);
+  A.kp = reinterpret_cast<int*>(A.ak + kmax_smem);
+  A.tab = reinterpret_cast<double2*>(A.kp + ((kmax_smem + 3) & ~3));
+  return A;
+}
 
 // duni (gcmc.f:2712-2805) with ir, jr and c held in registers across a run of draws; the
 // arithmetic is duni_next's, draw for draw.
@@ -317,48 +357,18 @@ __device__ __forceinline__ long long global_ns() {
   return (long long)t;
 }
 
-// One real-space candidate: a framework atom from a site's voxel list or a guest site.
-struct Cand {
-  double4 a;
-  int type, site;
-  bool live;
-};
-
-__device__ __forceinline__ Cand fetch_candidate(const DevSystem& S, const ChainDev& C, const MoveSmem& M, int nseg,
-                                                int t, int& s) {
-  Cand c;
-  c.live = false;
-  c.site = s;
-  if (t >= M.pre[M.nold + M.nnew]) return c;
-  while (t >= M.pre[s + 1]) s++;
-  c.site = s;
-  int j = t - M.pre[s];
-  if (j < M.vl[s]) {
-    c.a = S.vox_xyzq[M.vb[s] + j];
-    c.type = S.vox_type[M.vb[s] + j];
-    c.live = true;
-  } else {
-    int jg = j - M.vl[s], g = 0;
-    while (g + 1 < nseg && jg >= M.gpre[g + 1]) g++;
-    const int site_idx = C.seg_off[g] + (jg - M.gpre[g]);
-    if (site_idx < M.ex_lo || site_idx >= M.ex_hi) {
-      c.a = C.gsite[site_idx];
-      c.type = C.gtype[site_idx];
-      c.live = true;
-    }
-  }
-  return c;
-}
-
-// Warp 0: phase tables of the trial sites (ewald.f:95-137).
-__device__ __forceinline__ void build_phases(const DevSystem& S, const MoveSmem& M, void* tabv, int stride, int lane) {
-  const int nsite = M.nold + M.nnew, k1 = S.kmax[0], k2 = S.kmax[1];
+// Warp 0: phase tables of the trial sites (ewald.f:95-137).  The first axis carries the site's
+// charge, negative for a site that leaves, so that the reciprocal loop only multiplies and adds.
+__device__ __forceinline__ void build_phases(const SysConst& Y, const MoveSmem& M, double2* tab, int stride, int lane) {
+  const DevSystem& S = Y.S;
+  const int nold = M.nold, nsite = nold + M.nnew, k1 = S.kmax[0], k2 = S.kmax[1];
   for (int w = lane; w < nsite * 3; w += 32) {
     int st = w / 3, ax = w % 3;
     double f[3];
     frac_coords(S.cell, M.x[st], M.y[st], M.z[st], f);
     int off = st * stride + (ax == 0 ? 0 : (ax == 1 ? k1 + 1 : k1 + k2 + 2));
-    axis_phases(f[ax], S.kmax[ax], reinterpret_cast<double2*>(tabv) + off);
+    const double q = ax ? 1.0 : (st < nold ? -Y.sp[M.g].q[st] : Y.sp[M.g].q[st - nold]);
+    axis_phases(f[ax], S.kmax[ax], tab + off, q);
   }
 }
 
@@ -548,7 +558,7 @@ __device__ __forceinline__ void rotate_site(const double q[4], double& x, double
 // random_ins / random_disp + random_rot / random_jump), their charges and types, their voxel lists
 // and the real-space work list, then their phase tables (ewald.f:95-137).
 template <bool kProf>
-__device__ __noinline__ void build_trial(ChainDev& C, const SysConst& Y, const DevSystem& S, MoveSmem& M, void* tab,
+__device__ __noinline__ void build_trial(ChainDev& C, const SysConst& Y, const DevSystem& S, MoveSmem& M, double2* tab,
                                          int stride, int lane) {
   if (kProf && lane == 0) C.prof[8] -= clock64();
   const int mtype = M.mtype, ns = M.ns, nold = M.nold, nnew = M.nnew, nseg = Y.nspecies;
@@ -642,7 +652,7 @@ __device__ __noinline__ void build_trial(ChainDev& C, const SysConst& Y, const D
     M.x[lane] = ox;
     M.y[lane] = oy;
     M.z[lane] = oz;
-    M.q[lane] = P.q[lane];
+    M.cq[lane] = (nnew ? -P.q[lane] : P.q[lane]) * kR4pie0;
     M.type[lane] = P.type[lane];
     M.vb[lane] = vb_old;
     M.vl[lane] = vl_old;
@@ -652,25 +662,26 @@ __device__ __noinline__ void build_trial(ChainDev& C, const SysConst& Y, const D
     M.x[st] = nx;
     M.y[st] = ny;
     M.z[st] = nz;
-    M.q[st] = P.q[lane];
+    M.cq[st] = P.q[lane] * kR4pie0;
     M.type[st] = P.type[lane];
     const int v = voxel_of(S, nx, ny, nz);
     M.vb[st] = S.vox_off[v];
     M.vl[st] = S.vox_off[v + 1] - S.vox_off[v];
   }
   __syncwarp();
-  build_phases(S, M, tab, stride, lane);
-  // work-list prefix over the sites: each site's voxel list plus every guest site (warp scan)
+  build_phases(Y, M, tab, stride, lane);
+  // work-list prefix over the sites: each site's voxel list plus every guest site, in chunks of 32
+  // (warp scan)
   int gt = 0;
   for (int g = 0; g < nseg; g++) gt += C.nmol[g] * Y.sp[g].nsite;
-  int w = lane < nold + nnew ? M.vl[lane] + gt : 0;
+  int w = lane < nold + nnew ? (M.vl[lane] + gt + 31) >> 5 : 0;
   for (int o = 1; o < 32; o <<= 1) {
     const int u = __shfl_up_sync(0xffffffffu, w, o);
     if (lane >= o) w += u;
   }
-  if (lane < nold + nnew) M.pre[lane + 1] = w;
+  if (lane < nold + nnew) M.cpre[lane + 1] = w;
   if (lane == 0) {
-    M.pre[0] = 0;
+    M.cpre[0] = 0;
     int acc = 0;
     M.gpre[0] = 0;
     for (int g = 0; g < nseg; g++) {
@@ -681,145 +692,254 @@ __device__ __noinline__ void build_trial(ChainDev& C, const SysConst& Y, const D
   }
 }
 
-// Real-space sums of one pass: every (site, candidate) pair, compiled per boundary condition so
-// the hot loop holds one minimum-image form.  Deeper unrolling (2-8 candidates per trip) was
-// measured slower: the larger loop costs more in instruction fetch than it hides in latency.
-template <int kImcon, int NT, int CPT>
-__device__ __noinline__ void real_space(const DevSystem& S, const ChainDev& C, const MoveSmem& M, int nseg,
-                                        const int* prow_s, int nt1, double* vout) {
-  const int tid = threadIdx.x, nsite = M.nold + M.nnew, nold = M.nold, mtype = M.mtype;
-  double v1 = vout[1], v2 = vout[2];
-  const bool sub_old = (mtype != kInsert && mtype != kDelete);
-  const int T = M.pre[nsite];
-  // a thread takes candidates tid, tid + NT, tid + 2 NT, ... and adds them in that order;
-  // CPT candidates per loop trip, the next trip's loads issued before this one is evaluated
-  // (the pair's accumulation is written out in each loop: passing the candidate to a helper
-  // made ptxas spill in this loop)
-  if (CPT == 1) {
-    int s_next = 0;
-    Cand pre = fetch_candidate(S, C, M, nseg, tid, s_next);
-    for (int base = tid; base < T; base += NT) {
-      const Cand c = pre;
-      pre = fetch_candidate(S, C, M, nseg, base + NT, s_next);
-      if (!c.live) continue;
-      const int st = c.site;
-      const int row = prow_s[M.type[st] * nt1 + c.type];
-      double ec = 0.0, ev = 0.0;
-      pair_energy<kImcon>(S, M.x[st] - c.a.x, M.y[st] - c.a.y, M.z[st] - c.a.z, M.q[st] * kR4pie0, c.a.w, row, ec,
-                          ev);
-      if (sub_old && st < nold) {
-        v1 -= ec;
-        v2 -= ev;
-      } else {
-        v1 += ec;
-        v2 += ev;
-      }
-    }
-  } else {
-    int s0 = 0, s1 = 0;
-    Cand p0 = fetch_candidate(S, C, M, nseg, tid, s0);
-    Cand p1 = fetch_candidate(S, C, M, nseg, tid + NT, s1);
-    for (int base = tid; base < T; base += 2 * NT) {
-      const Cand c0 = p0, c1 = p1;
-      p0 = fetch_candidate(S, C, M, nseg, base + 2 * NT, s0);
-      p1 = fetch_candidate(S, C, M, nseg, base + 3 * NT, s1);
-      if (c0.live) {
-        const int st = c0.site;
-        const int row = prow_s[M.type[st] * nt1 + c0.type];
-        double ec = 0.0, ev = 0.0;
-        pair_energy<kImcon>(S, M.x[st] - c0.a.x, M.y[st] - c0.a.y, M.z[st] - c0.a.z, M.q[st] * kR4pie0, c0.a.w, row,
-                            ec, ev);
-        if (sub_old && st < nold) {
-          v1 -= ec;
-          v2 -= ev;
-        } else {
-          v1 += ec;
-          v2 += ev;
-        }
-      }
-      if (c1.live) {
-        const int st = c1.site;
-        const int row = prow_s[M.type[st] * nt1 + c1.type];
-        double ec = 0.0, ev = 0.0;
-        pair_energy<kImcon>(S, M.x[st] - c1.a.x, M.y[st] - c1.a.y, M.z[st] - c1.a.z, M.q[st] * kR4pie0, c1.a.w, row,
-                            ec, ev);
-        if (sub_old && st < nold) {
-          v1 -= ec;
-          v2 -= ev;
-        } else {
-          v1 += ec;
-          v2 += ev;
-        }
-      }
-    }
-  }
-  vout[1] = v1;
-  vout[2] = v2;
+// ------------------------------------------------------------------ energy sums of a trial
+// A thread's share of the reciprocal change (ewald.f:139-331): S_new(k) = S(k) + dS(k) to Sn, and akk
+// and |S_new|^2 - |S|^2 (ewald.f:311-319) returned.  A thread takes k-vectors tid, tid + NT, ... and adds their terms in that
+// order, KPT of them in flight.  Bound by the latency of its shared-memory reads and FP64 chain with
+// 1-4 k-vectors a thread, so the site loop is unrolled and the products go straight into the sums.
+__device__ __forceinline__ double flip_sign(double v, int mask) {
+  return __hiloint2double(__double2hiint(v) ^ mask, __double2loint(v));
 }
 
-// All threads: this thread's share of the reciprocal sum (v[0] = sum akk*d|S|^2) and of the
-// real-space pairs (v[1] ewld2, v[2] vdw); S_new goes to Sn.
-// One k-vector's change: S_new(k) from S(k) and the trial sites' phases; returns
-// akk (|S_new|^2 - |S_old|^2).
-__device__ __forceinline__ double recip_term(int k, const MoveSmem& M, const int* kp, const double* ak,
-                                             const double2* Sk, double2* Sn, const double2* tb, int stride, int k1,
-                                             int k2) {
-  const int nsite = M.nold + M.nnew, nold = M.nold, mtype = M.mtype;
+// Sums over sites and k-vectors are written as fma: what the compiler contracts may differ between
+// the kernel's compiled tiles, which agree bit for bit.
+__device__ __forceinline__ double2 recip_term(int k, int nsite, int k1, int k2, int stride, const double2* tb,
+                                             const int* kp, const double* ak, const double2* Sk, double2* Sn) {
   int l, m, n;
   kunpack(kp[k], l, m, n);
-  int am = m < 0 ? -m : m, an = n < 0 ? -n : n;
-  double2 so = Sk[k], sn;
-  double2 aold = make_double2(0.0, 0.0), anew = make_double2(0.0, 0.0);
-  for (int st = 0; st < nsite; st++) {
-    const double2* t = tb + st * stride;
-    double2 c = m >= 0 ? cmul(t[l], t[k1 + 1 + am]) : cmulc(t[l], t[k1 + 1 + am]);
-    c = n >= 0 ? cmul(c, t[k1 + k2 + 2 + an]) : cmulc(c, t[k1 + k2 + 2 + an]);
-    double q = M.q[st];
-    if (st < nold) {
-      aold.x += q * c.x;
-      aold.y += q * c.y;
-    } else {
-      anew.x += q * c.x;
-      anew.y += q * c.y;
-    }
+  const int o2 = k1 + 1 + (m < 0 ? -m : m), o3 = k1 + k2 + 2 + (n < 0 ? -n : n);
+  const int sm = m & 0x80000000, sn = n & 0x80000000;
+  double ax = 0.0, ay = 0.0;
+  const double2* t = tb;
+#pragma unroll 3
+  for (int st = 0; st < nsite; st++, t += stride) {
+    const double2 e1 = t[l], e2 = t[o2], e3 = t[o3];
+    const double y2 = flip_sign(e2.y, sm), y3 = flip_sign(e3.y, sn);
+    const double cx = fma(-e1.y, y2, e1.x * e2.x), cy = fma(e1.x, y2, e1.y * e2.x);
+    ax = fma(cx, e3.x, ax);
+    ay = fma(cy, e3.x, ay);
+    ax = fma(-cy, y3, ax);
+    ay = fma(cx, y3, ay);
   }
-  if (mtype == kInsert)
-    sn = make_double2(anew.x + so.x, anew.y + so.y);
-  else if (mtype == kDelete)
-    sn = make_double2(so.x - aold.x, so.y - aold.y);
-  else
-    sn = make_double2((so.x - aold.x) + anew.x, (so.y - aold.y) + anew.y);
-  Sn[k] = sn;
-  return ak[k] * (sn.x * sn.x + sn.y * sn.y - so.x * so.x - so.y * so.y);
+  const double2 so = Sk[k], sw = make_double2(so.x + ax, so.y + ay);
+  Sn[k] = sw;
+  return make_double2(ak[k], sw.x * sw.x + sw.y * sw.y - so.x * so.x - so.y * so.y);
 }
 
-// All threads: this thread's share of the reciprocal sum (v[0] = sum akk*d|S|^2) and of the
-// real-space pairs (v[1] ewld2, v[2] vdw); S_new goes to Sn.  A thread takes k-vectors tid,
-// tid + NT, ... and adds their terms in that order, KPT of them per trip.
-template <int NT, int KPT, int CPT>
-__device__ __noinline__ void sums(const DevSystem& S, const ChainDev& C, const MoveSmem& M, int nseg, const int* prow_s,
-                                  int nt1, const int* kp, const double* ak, const double2* Sk, double2* Sn,
-                                  const void* tabv, int stride, double* v) {
-  const int tid = threadIdx.x, K = S.K, k1 = S.kmax[0], k2 = S.kmax[1];
-  const double2* tb = reinterpret_cast<const double2*>(tabv);
-  if (KPT == 1) {
-    for (int k = tid; k < K; k += NT) v[0] += recip_term(k, M, kp, ak, Sk, Sn, tb, stride, k1, k2);
-  } else {
-    int k = tid;
-    for (; k + NT < K; k += 2 * NT) {  // two independent k-vectors in flight, added in order
-      v[0] += recip_term(k, M, kp, ak, Sk, Sn, tb, stride, k1, k2);
-      v[0] += recip_term(k + NT, M, kp, ak, Sk, Sn, tb, stride, k1, k2);
+// How a chunk's pairs are imaged and tabulated, compiled separately so that the loop holds one form
+// (each copy costs instruction cache): orthorhombic cells (imcon 1, 2) and parallelepipeds (3) with
+// one table spacing, and everything else (half-shift cells, slabs, rvdw other than rcut) reading the
+// boundary condition from the cell.
+enum PairKind : int { kPairOrtho = 0, kPairTriclinic = 1, kPairGeneral = 2 };
+
+// One candidate of a chunk: its atom and type (-1: none in this lane), and the trial site the chunk
+// belongs to (the same for every lane).
+struct Cand {
+  double x, y, z, q;
+  int type, site;
+};
+
+__device__ __forceinline__ void load_site(const double4* p, Cand& c) {
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(c.x), "=d"(c.y), "=d"(c.z), "=d"(c.q) : "l"(p));
+}
+
+// Chunk `chunk` of the work list: 32 candidates of one site.  `incl` is lane s's inclusive chunk
+// prefix of site s, so the site is the number of lanes whose prefix the chunk has passed.
+__device__ __forceinline__ void load_chunk(const BatchSmem& B, int chunk, int nchunk, int incl, int gt, Cand& c) {
+  const MoveSmem& M = B.M;
+  const DevSystem& S = B.Y.S;
+  c.x = c.y = c.z = c.q = 0.0;
+  c.type = -1;
+  c.site = 0;
+  if (chunk >= nchunk) return;  // the whole warp
+  const int s = __popc(__ballot_sync(0xffffffffu, chunk >= incl));
+  c.site = s;
+  const int j = ((chunk - M.cpre[s]) << 5) + (threadIdx.x & 31), vl = M.vl[s];
+  if (j < vl) {
+    const int i = M.vb[s] + j;
+    load_site(S.vox_xyzq + i, c);
+    c.type = S.vox_type[i];
+  } else if (j - vl < gt) {
+    const int jg = j - vl;
+    int g = 0;
+    while (g + 1 < B.Y.nspecies && jg >= M.gpre[g + 1]) g++;
+    const int i = B.C.seg_off[g] + (jg - M.gpre[g]);
+    if (i < M.ex_lo || i >= M.ex_hi) {
+      load_site(B.C.gsite + i, c);
+      c.type = B.C.gtype[i];
     }
-    if (k < K) v[0] += recip_term(k, M, kp, ak, Sk, Sn, tb, stride, k1, k2);
   }
-  // real space, per boundary condition
-  if (S.cell.imcon == 1) real_space<1, NT, CPT>(S, C, M, nseg, prow_s, nt1, v);
-  else if (S.cell.imcon == 2) real_space<2, NT, CPT>(S, C, M, nseg, prow_s, nt1, v);
-  else if (S.cell.imcon == 3) real_space<3, NT, CPT>(S, C, M, nseg, prow_s, nt1, v);
-  // the half-shift cells and the slab share one instantiation that reads the boundary condition
-  // from the cell: each compiled copy of this loop costs instruction cache (one per cell kind
-  // cost 8%)
-  else real_space<-1, NT, CPT>(S, C, M, nseg, prow_s, nt1, v);
+}
+
+// This warp's share of the real-space pairs (ewald2 + srfrce over guestlistgen's set): chunks warp,
+// warp + NW, ... of the work list, each lane adding its pairs in that order.  The loop is bound by
+// latency (two chains, 16 warps, share an SM): a pair is a candidate load, an image, a root, three
+// table reads and two interpolations, each waiting for the last.  So U chunks are in flight: their
+// distances first, then the next U chunks' loads, then their table reads, without a branch in
+// between -- a lane whose candidate is missing or beyond the cut-off reads the table at the cut-off
+// and adds zero.  Energy sums of a move, SM cycles (256 chains of 16 frameworks, 1 A voxels, two
+// chains on most SMs; one chain alone on its SM): 17.8k; 12.6k with one branching candidate a trip and
+// two separate tables, 10.5k; 7.4k with U = 2, 10.9k; 7.5k with 3, 11.2k; 8.1k with 4.
+template <int KIND, int NT, int U>
+__device__ __forceinline__ void real_space(const BatchSmem& B, double& v1, double& v2) {
+  const MoveSmem& M = B.M;
+  const DevSystem& S = B.Y.S;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, NW = NT / 32;
+  const int nold = M.nold, nsite = nold + M.nnew, gt = M.gpre[B.Y.nspecies];
+  const int nchunk = M.cpre[nsite], nt1 = S.ntypes + 1;
+  const int incl = lane < nsite ? M.cpre[lane + 1] : 0x7fffffff;
+  const bool sub_old = M.mtype != kInsert && M.mtype != kDelete;
+  const double rcut2 = S.rcut2, rdr = S.rdr_e, rdrv = S.rdr_v;
+  const int tstride = S.tab_stride;
+  // imcon 1 takes the first edge for every axis (images, utility_pack.f:1138-1349)
+  const int iy = S.cell.imcon == 1 ? 0 : 1, iz = S.cell.imcon == 1 ? 0 : 2;
+  const double hx = S.cell.h[0], hy = S.cell.h[4 * iy], hz = S.cell.h[4 * iz];
+  const double rx = S.cell.inv[0], ry = S.cell.inv[iy], rz = S.cell.inv[iz];
+  constexpr double kMagic = 6755399441055744.0;  // 1.5 x 2^52: adding it rounds to an integer
+  Cand c[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) load_chunk(B, warp + u * NW, nchunk, incl, gt, c[u]);
+  for (int base = warp; base < nchunk; base += U * NW) {
+    double rs[U], cq[U], sg[U];
+    int off[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int s = c[u].site;
+      double dx = M.x[s] - c[u].x, dy = M.y[s] - c[u].y, dz = M.z[s] - c[u].z;
+      if (KIND == kPairOrtho) {
+        // nint by the rounding of an addition: a tie picks either image, at the same distance
+        dx = fma(-hx, (fma(rx, dx, kMagic) - kMagic), dx);
+        dy = fma(-hy, (fma(ry, dy, kMagic) - kMagic), dy);
+        dz = fma(-hz, (fma(rz, dz, kMagic) - kMagic), dz);
+      } else if (KIND == kPairTriclinic) {
+        min_image_t<3>(S.cell, dx, dy, dz);
+      } else {
+        min_image(S.cell, dx, dy, dz);
+      }
+      const double rsq = fma(dx, dx, fma(dy, dy, dz * dz));
+      const bool in = c[u].type >= 0 && rsq < rcut2;
+      const double qq = M.cq[s] * c[u].q;
+      rs[u] = in ? rsq : rcut2;
+      cq[u] = in && fabs(qq) > 1e-10 ? qq : 0.0;  // ewald2 skips smaller products
+      const int row = in ? B.prow[M.type[s] * nt1 + c[u].type] : -1;
+      off[u] = row > 0 ? row * tstride : 0;
+      sg[u] = row < 0 ? 0.0 : (sub_old && s < nold ? -1.0 : 1.0);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) load_chunk(B, base + (U + u) * NW, nchunk, incl, gt, c[u]);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const double r = sqrt_approx(rs[u]);
+      const double x = __dmul_rn(r, rdr);
+      const double t = (x - 0.5) + kMagic;  // floor(x) but for integers, where either interval agrees
+      const int l = __double2loint(t);
+      const double p = x - (t - kMagic), pm = p - 1.0, hp = 0.5 * p;
+      if (KIND != kPairGeneral) {
+        const double2* tb = S.pair_tab + (off[u] + l);
+        const double2 a0 = tb[0], a1 = tb[1], a2 = tb[2];
+        const double e1 = fma(a1.x - a0.x, p, a0.x), e2 = fma(a2.x - a1.x, pm, a1.x);
+        const double w1 = fma(a1.y - a0.y, p, a0.y), w2 = fma(a2.y - a1.y, pm, a1.y);
+        v1 = fma(fma(e2 - e1, hp, e1), cq[u], v1);
+        v2 = fma(fma(w2 - w1, hp, w1), sg[u], v2);
+      } else {
+        v1 = fma(interp3(S.erc, r, rdr), cq[u], v1);
+        if (sg[u] != 0.0) v2 = fma(interp3(S.vvv + off[u], r, rdrv), sg[u], v2);
+      }
+    }
+  }
+}
+
+// The rotation of a single-site molecule changes no energy: what is left of E_new - E_old is the
+// rounding of two sums of the same pairs, yet its sign decides whether the acceptance test draws a
+// random number (gcmc.f:1330-1338).  So that seeded trajectories of uncharged molecules of that kind
+// stay what they are, these pairs keep one fixed arithmetic and order of addition: candidates tid, tid + NT, ... of the
+// old site's list and guests, then the new site's, correctly rounded roots, one table at a time.
+template <int NT>
+__device__ __noinline__ void real_space_residue(double* vout) {
+  const BatchSmem& B = batch_smem();
+  const MoveSmem& M = B.M;
+  const DevSystem& S = B.Y.S;
+  const int gt = M.gpre[B.Y.nspecies], T0 = M.vl[0] + gt, T = T0 + M.vl[1] + gt, nt1 = S.ntypes + 1;
+  const double chgea = B.Y.sp[M.g].q[0] * kR4pie0;
+  double v1 = 0.0, v2 = 0.0;
+  for (int t = threadIdx.x; t < T; t += NT) {
+    const int s = t >= T0, j = t - (s ? T0 : 0);
+    double4 a;
+    int type;
+    if (j < M.vl[s]) {
+      a = S.vox_xyzq[M.vb[s] + j];
+      type = S.vox_type[M.vb[s] + j];
+    } else {
+      const int jg = j - M.vl[s];
+      int g = 0;
+      while (g + 1 < B.Y.nspecies && jg >= M.gpre[g + 1]) g++;
+      const int i = B.C.seg_off[g] + (jg - M.gpre[g]);
+      if (i >= M.ex_lo && i < M.ex_hi) continue;
+      a = B.C.gsite[i];
+      type = B.C.gtype[i];
+    }
+    const int row = B.prow[M.type[s] * nt1 + type];
+    double ec = 0.0, ev = 0.0;
+    pair_energy(S, M.x[s] - a.x, M.y[s] - a.y, M.z[s] - a.z, chgea, a.w, row, ec, ev);
+    if (s == 0) {
+      v1 -= ec;
+      v2 -= ev;
+    } else {
+      v1 += ec;
+      v2 += ev;
+    }
+  }
+  vout[0] = v1;
+  vout[1] = v2;
+}
+
+// Every thread: its share of {sum akk d|S|^2, ewld2, vdw}, summed over its warp into red.
+template <int KIND, int NT, int KPT, int CPT>
+__device__ __noinline__ void sums_kind(int kmax_smem, int stride) {
+  BatchSmem& B = batch_smem();
+  const BatchArrays A = batch_arrays(kmax_smem);
+  const DevSystem& S = B.Y.S;
+  const int tid = threadIdx.x, K = S.K, k1 = S.kmax[0], k2 = S.kmax[1], nsite = B.M.nold + B.M.nnew;
+  double v0 = 0.0, v1 = 0.0, v2 = 0.0;
+  auto term = [&](int k) { return recip_term(k, nsite, k1, k2, stride, A.tab, A.kp, A.ak, A.Sk, A.Sn); };
+  int k = tid;
+  if (KPT == 2)
+    for (; k + NT < K; k += 2 * NT) {  // two independent k-vectors in flight, added in order
+      const double2 a = term(k), b = term(k + NT);
+      v0 = fma(b.x, b.y, fma(a.x, a.y, v0));
+    }
+  for (; k < K; k += NT) {
+    const double2 a = term(k);
+    v0 = fma(a.x, a.y, v0);
+  }
+  if (B.M.ns == 1 && B.M.mtype == kRotate) {
+    double v[2];
+    real_space_residue<NT>(v);
+    v1 = v[0];
+    v2 = v[1];
+  } else {
+    real_space<KIND, NT, kChunksPerTrip * CPT>(B, v1, v2);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    v0 += __shfl_down_sync(0xffffffffu, v0, o);
+    v1 += __shfl_down_sync(0xffffffffu, v1, o);
+    v2 += __shfl_down_sync(0xffffffffu, v2, o);
+  }
+  if ((tid & 31) == 0) {
+    double* red = B.red + 3 * (tid >> 5);
+    red[0] = v0;
+    red[1] = v1;
+    red[2] = v2;
+  }
+}
+
+template <int NT, int KPT, int CPT>
+__device__ __forceinline__ void sums(const DevSystem& S, int kmax_smem, int stride) {
+  const int imcon = S.cell.imcon;
+  if (S.pair_tab && imcon <= 2) sums_kind<kPairOrtho, NT, KPT, CPT>(kmax_smem, stride);
+  else if (S.pair_tab && imcon == 3) sums_kind<kPairTriclinic, NT, KPT, CPT>(kmax_smem, stride);
+  else sums_kind<kPairGeneral, NT, KPT, CPT>(kmax_smem, stride);
 }
 
 // All threads, in production: storeprob (utility_pack.f:496-561) for the chain's state after the
@@ -866,12 +986,10 @@ __device__ __noinline__ void prob_store(const SysConst& Y, const ChainDev& C) {
 template <bool kProf, int NT, int KPT, int CPT>
 __global__ void __launch_bounds__(NT, NT <= 128 ? 4 : (NT <= 256 ? 2 : 1)) fmc_batch_kernel(BatchLaunch L,
                                                                                            int tab_stride) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ ChainDev C;
-  __shared__ MoveSmem M;
-  __shared__ SysConst Ysm;
-  __shared__ double red[32 * 3];
-  __shared__ int prow_s[(kBatchMaxTypes + 1) * (kBatchMaxTypes + 1)];
+  BatchSmem& B = batch_smem();
+  ChainDev& C = B.C;
+  MoveSmem& M = B.M;
+  SysConst& Ysm = B.Y;
   DevSystem& S = Ysm.S;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if ((int)blockIdx.x >= L.nchains) return;
@@ -891,18 +1009,15 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 4 : (NT <= 256 ? 2 : 1)) fmc_b
   }
   __syncthreads();
   const SysConst& Y = Ysm;
-  const int K = S.K, Kmax = L.kmax_smem, nseg = Y.nspecies;
+  const int K = S.K, kmax_smem = L.kmax_smem;
   const int nt1 = S.ntypes + 1;
-  for (int i = tid; i < nt1 * nt1; i += blockDim.x) prow_s[i] = S.pair_row[i];
-  double2* Sk = reinterpret_cast<double2*>(smem_raw);
-  double2* Sn = Sk + Kmax;
-  double* ak = reinterpret_cast<double*>(Sn + Kmax);
-  int* kp = reinterpret_cast<int*>(ak + Kmax);
-  void* tab = reinterpret_cast<void*>(kp + ((Kmax + 3) & ~3));
+  for (int i = tid; i < nt1 * nt1; i += blockDim.x) B.prow[i] = S.pair_row[i];
+  const BatchArrays A = batch_arrays(kmax_smem);
+  double2 *const Sk = A.Sk, *const Sn = A.Sn, *const tab = A.tab;
   for (int k = tid; k < K; k += blockDim.x) {
     Sk[k] = C.sk[k];
-    ak[k] = S.akk[k];
-    kp[k] = S.kpack[k];
+    A.ak[k] = S.akk[k];
+    A.kp[k] = S.kpack[k];
   }
   const int stride = S.kmax[0] + S.kmax[1] + S.kmax[2] + 3;
   (void)tab_stride;
@@ -935,16 +1050,18 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 4 : (NT <= 256 ? 2 : 1)) fmc_b
     }
     if (C.status) break;
     const bool last = !C.lgchk;  // lane 0 of warp 0 writes lgchk only in select_move
-    double v[3] = {0.0, 0.0, 0.0};
-    sums<NT, KPT, CPT>(S, C, M, nseg, prow_s, nt1, kp, ak, Sk, Sn, tab, stride, v);
+    sums<NT, KPT, CPT>(S, kmax_smem, stride);
     if (prof && tid == 0) C.prof[6] += clock64() - t0;
-    block_sum<3>(v, red);
+    __syncthreads();
     if (prof && tid == 0) {
       t1 = clock64();
       C.prof[2] += t1 - t0;
       t0 = t1;
     }
     if (tid == 0) {
+      double v[3] = {0.0, 0.0, 0.0};
+      for (int w = 0; w < NT / 32; w++)
+        for (int k = 0; k < 3; k++) v[k] += B.red[3 * w + k];
       assemble(Y, M, v);
       decide(C, Y, M);
     }
@@ -987,7 +1104,7 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 4 : (NT <= 256 ? 2 : 1)) fmc_b
         }
       } else if (tid < ns) {
         int st = (mtype == kInsert) ? tid : ns + tid;
-        C.gsite[M.commit_lo + tid] = make_double4(M.x[st], M.y[st], M.z[st], M.q[st]);
+        C.gsite[M.commit_lo + tid] = make_double4(M.x[st], M.y[st], M.z[st], Y.sp[M.g].q[tid]);
         C.gtype[M.commit_lo + tid] = M.type[st];
       }
     }
@@ -1022,8 +1139,8 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 4 : (NT <= 256 ? 2 : 1)) fmc_b
 }  // namespace
 
 int batch_smem_bytes(int kmax_K, int tab_sites, int tab_stride) {
-  return kmax_K * (int)(2 * sizeof(double2) + sizeof(double)) + ((kmax_K + 3) & ~3) * (int)sizeof(int) +
-         tab_sites * tab_stride * (int)sizeof(double2);
+  return kBatchSmemBytes + kmax_K * (int)(2 * sizeof(double2) + sizeof(double)) +
+         ((kmax_K + 3) & ~3) * (int)sizeof(int) + tab_sites * tab_stride * (int)sizeof(double2);
 }
 
 namespace {

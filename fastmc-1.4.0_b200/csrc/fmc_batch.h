@@ -25,6 +25,8 @@ constexpr int kBatchMaxTab = kBatchMaxTypes * (kBatchMaxTypes + 1) / 2;
 struct BatchTile {
   int threads, kvec_per_trip, cand_per_trip;
 };
+// Chunks of 32 candidates a warp has in flight in the real-space loop, per candidate of the tile.
+constexpr int kChunksPerTrip = 2;
 constexpr int kNumBatchTiles = 12;
 constexpr BatchTile kBatchTiles[kNumBatchTiles] = {
     {256, 1, 1}, {256, 2, 1}, {256, 1, 2}, {256, 2, 2}, {128, 1, 1}, {128, 2, 1},

@@ -105,6 +105,13 @@ int upload_system(const HostSystem& h, DeviceSystem& d, std::string& err) {
   if ((e = upload(d.allocations, &v.erc, h.erc)) != cudaSuccess) goto fail;
   if ((e = upload(d.allocations, &v.vvv, h.vvv)) != cudaSuccess) goto fail;
   v.tab_stride = h.mxgrid + 1;
+  if (v.rdr_e == v.rdr_v) {
+    double2* pt = nullptr;
+    if ((e = dalloc(d.allocations, &pt, h.vvv.size())) != cudaSuccess) goto fail;
+    if ((e = launch_pack_tables(v.erc, v.vvv, v.tab_stride, h.ntables + 1, pt, 0)) != cudaSuccess) goto fail;
+    if ((e = cudaStreamSynchronize(0)) != cudaSuccess) goto fail;
+    v.pair_tab = pt;
+  }
   v.ntypes = h.ntypes;
   if ((e = upload(d.allocations, &v.pair_row, h.pair_row)) != cudaSuccess) goto fail;
   v.K = h.K;

@@ -554,6 +554,18 @@ FMC_HD void window_close(WindowStats& W, int ng, int nwind, double temp, CS cs) 
   W.rollcount = 0;
 }
 
+// Square root of x > 0 from y, an estimate of 1/sqrt(x) good to about 20 bits: one coupled
+// Goldschmidt step for sqrt(x) and 1/(2 sqrt(x)), then a Newton correction of the root by its
+// exact residual (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990), within an ulp of sqrt(x).  No branch, so that several roots stay in flight.
+FMC_HD double sqrt_refine(double x, double y) {
+  double g = x * y, h = 0.5 * y;
+  const double r = fma(-h, g, 0.5);
+  g = fma(g, r, g);
+  h = fma(h, r, h);
+  return fma(fma(-g, g, x), h, g);
+}
+
 // 3-point interpolation of a tabulated function on r_l = l*dr (ewald.f:670-684,
 // vdw_terms.f:476-489).  tab[0] is defined as tab[1].
 FMC_HD double interp3(const double* tab, double rrr, double rdr) {

@@ -28,6 +28,9 @@ struct DevSystem {
   double rcut2, rdr_e, rdr_v;
   const double* erc;
   const double* vvv;
+  // {erc, vvv} of one table row interleaved, row 0 holding {erc, 0} for pairs without a vdW
+  // table; null when the two tables have different spacings (rvdw other than rcut)
+  const double2* pair_tab;
   int tab_stride;
   int ntypes;
   const int* pair_row;
@@ -65,16 +68,26 @@ __device__ __forceinline__ double2 cmulc(double2 a, double2 b) {  // a * conj(b)
   return make_double2(a.x * b.x + a.y * b.y, a.y * b.x - b.y * a.x);
 }
 
-// e^{i 2 pi j s} for j = 0..kmax by the recurrence of ewald.f:118-137 into tab[0..kmax].
-__device__ __forceinline__ void axis_phases(double s, int kmax, double2* tab) {
+// q e^{i 2 pi j s} for j = 0..kmax by the recurrence of ewald.f:118-137 into tab[0..kmax].
+__device__ __forceinline__ void axis_phases(double s, int kmax, double2* tab, double q = 1.0) {
   double sn, cs;
   sincos(2.0 * kPi * s, &sn, &cs);
-  tab[0] = make_double2(1.0, 0.0);
-  if (kmax >= 1) tab[1] = make_double2(cs, sn);
+  tab[0] = make_double2(q, 0.0);
+  double2 p = make_double2(q * cs, q * sn);
+  if (kmax >= 1) tab[1] = p;
   for (int j = 2; j <= kmax; j++) {
-    double2 p = tab[j - 1];
-    tab[j] = make_double2(p.x * cs - p.y * sn, p.y * cs + p.x * sn);
+    p = make_double2(p.x * cs - p.y * sn, p.y * cs + p.x * sn);
+    tab[j] = p;
   }
+}
+
+// sqrt(x) for x >= 0 without a branch: the hardware's estimate of 1/sqrt(x), refined.  The added
+// 1e-300 leaves every normal x as it is and keeps x = 0 finite.
+__device__ __forceinline__ double sqrt_approx(double x) {
+  double y;
+  x += 1e-300;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return sqrt_refine(x, y);
 }
 
 // Fractional coordinates s = rcell . r as in ewald.f:106-108.

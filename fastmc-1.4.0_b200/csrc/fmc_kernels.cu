@@ -764,6 +764,22 @@ __global__ void __launch_bounds__(kScanThreads) fmc_exclusive_scan_kernel(const 
 }
 }  // namespace
 
+namespace {
+__global__ void __launch_bounds__(256) fmc_pack_tables_kernel(const double* __restrict__ erc,
+                                                              const double* __restrict__ vvv, int stride, int n,
+                                                              double2* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = make_double2(erc[i % stride], i < stride ? 0.0 : vvv[i]);
+}
+}  // namespace
+
+cudaError_t launch_pack_tables(const double* erc, const double* vvv, int stride, int rows, double2* out,
+                               cudaStream_t st) {
+  const int n = rows * stride;
+  if (n > 0) fmc_pack_tables_kernel<<<(n + 255) / 256, 256, 0, st>>>(erc, vvv, stride, n, out);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_exclusive_scan(const int* counts, int n, int* off, cudaStream_t st) {
   fmc_exclusive_scan_kernel<<<1, kScanThreads, 0, st>>>(counts, n, off);
   return cudaGetLastError();

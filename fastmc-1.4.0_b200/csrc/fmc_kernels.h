@@ -112,6 +112,10 @@ cudaError_t launch_voxel_fill(const CellGeom& cell, const int* nvox, const doubl
                               double lim2, const unsigned* code, const int* off, int* atoms, unsigned short* atoms16,
                               double4* xyzq, unsigned char* vtype, long long cap,
                               cudaStream_t st);  // entries >= cap not written
+// The {erc, vvv} rows of DevSystem::pair_tab: rows * stride entries, row r holding vvv's row r
+// (row 0: no vdW table).
+cudaError_t launch_pack_tables(const double* erc, const double* vvv, int stride, int rows, double2* out,
+                               cudaStream_t st);
 // off[0..n]: exclusive prefix sum of counts[0..n-1], off[n] the total (one CTA)
 cudaError_t launch_exclusive_scan(const int* counts, int n, int* off, cudaStream_t st);
 

@@ -185,13 +185,14 @@ int build_slot(const HostSystem& h, int slot, const int seed[4], SlotMemory& mem
   double4* xyzq = nullptr;
   unsigned char* vt = nullptr;
   double2* skfw = nullptr;
+  double2* ptab = nullptr;
   double* scratch = nullptr;
   double* parts = nullptr;
   {
     // every buffer of the slot, set-up scratch included, from one pool allocation
     const size_t arena = total + al(sizeof(int) * nv) + (prefilter ? al(sizeof(unsigned) * h.nf) : 0) +
                          al(sizeof(int) * (nv + 1)) + al(sizeof(double4) * vox_cap) + al(vox_cap) +
-                         al(sizeof(double2) * std::max(h.K, 1)) +
+                         al(sizeof(double2) * std::max(h.K, 1)) + al(sizeof(double2) * h.vvv.size()) +
                          al(sizeof(double) * std::max<size_t>(recip_scratch_doubles(v, h.nf), 1)) +
                          al(sizeof(double) * (recip_nparts(v) + 1)) + chain_state_bytes(h.deck, h, true) + 16 * 256;
     if ((e = mem.reserve(arena)) != cudaSuccess) goto fail;
@@ -229,6 +230,11 @@ int build_slot(const HostSystem& h, int slot, const int seed[4], SlotMemory& mem
   v.rdr_e = 1.0 / h.drewd;
   v.rdr_v = 1.0 / h.dlrpot;
   v.tab_stride = h.mxgrid + 1;
+  if (v.rdr_e == v.rdr_v) {
+    if ((e = mem.alloc((void**)&ptab, sizeof(double2) * h.vvv.size())) != cudaSuccess) goto fail;
+    if ((e = launch_pack_tables(v.erc, v.vvv, v.tab_stride, h.ntables + 1, ptab, st)) != cudaSuccess) goto fail;
+    v.pair_tab = ptab;
+  }
   v.ntypes = h.ntypes;
   v.recip_pref = h.recip_pref;
   // framework S(k)
