@@ -1,13 +1,19 @@
 // Persistent batched kernel: one CTA (256 threads) per chain runs `moves` iterations of the
 // move loop (gcmc.f:589-1380) entirely on the device.
 //
-// Per move: thread 0 draws the random numbers, picks and builds the trial (duni, move choice,
-// step-size adaptation, random_ins / random_disp), all threads then build the trial sites'
-// phase tables in shared memory, sweep their k-vectors (S(k), S_new, akk and the k-vector table
-// are resident in shared memory for the whole launch) and their share of the real-space pair
-// candidates (framework voxel list + guest sites), one fixed-order block reduction gives
-// {sum akk*d|S|^2, ewld2, vdw}, thread 0 applies energy_eval, and on acceptance every thread
-// commits its own k-vectors while the block updates the guest-site segment.
+// Per move: four warps set the move up side by side -- warp 0 takes the draws, chooses the move and
+// builds the trial sites and the real-space work list, warp 1 finishes the last move's bookkeeping,
+// warp 2 builds the phase tables, warp 3 the tail correction -- then all threads sweep their k-vectors
+// (S(k), S_new, akk and the k-vector table are resident in shared memory for the whole launch) and
+// their share of the real-space pair candidates, and every thread applies energy_eval to the warps'
+// sums and commits its own k-vectors: two block barriers a move.
+//
+// A chain's move is a serial chain of latencies; what one costs, in SM cycles (16 chains, one an SM,
+// K = 131, 510 atoms / 256 chains of 16 frameworks, two chains on most SMs): before the set-up and the
+// bookkeeping were split over warps 24.2k / 30.8k (set-up 7.0k / 8.3k, sums 12.6k / 17.6k, acceptance,
+// bookkeeping and commit 4.6k / 4.9k), now 14.5k / 20.6k.  Code that runs once a move comes through the
+// instruction caches (32 KB, then 128 KB) each time, at up to ten cycles an instruction, so the set-up
+// keeps one path for every move type and its rare parts out of line.
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -18,28 +24,43 @@ namespace fmc {
 
 namespace {
 
+// The trial being evaluated: what the energy sums read, written while the move is set up.
 struct MoveSmem {
-  int mtype, g, mol, nold, nnew, accepted, ex_lo, ex_hi;
-  int commit_lo, seg_end, ns, randchoice, need_lrc, rande_drawn;
-  double delrc, rande;
+  int mtype, g, nold, nnew, ns, ex_lo, ex_hi;
   double r[7], dis_delr, dis_rot;  // the trial's random numbers and step sizes (select_move)
-  double ewld1, ewld2, vdw, ewld3, estep;
   // trial sites (old ones first): position, charge factor q r4pie0 (negative for the old sites of a
-  // displacement, whose energies are subtracted) and atom type
+  // displacement, whose energies are subtracted) and atom type, times types + 1 (a row of prow)
   double x[2 * kBatchMaxSites], y[2 * kBatchMaxSites], z[2 * kBatchMaxSites], cq[2 * kBatchMaxSites];
   int type[2 * kBatchMaxSites];
-  // real-space work list: per trial site its voxel-list start/length and the prefix over the sites
-  // of its chunks of 32 candidates (voxel entries, then every guest site)
-  int vb[2 * kBatchMaxSites], vl[2 * kBatchMaxSites], cpre[2 * kBatchMaxSites + 1];
-  int gpre[kMaxGuestTypes + 1];
+  // real-space work list, in chunks of 32 candidates: entry e < nsite is trial site e's voxel list {chunks
+  // before it, first entry, length} (nfw chunks in all), entry nsite + e every guest site for it (gchunks)
+  int4 list[2 * kBatchMaxSites];
+  int nfw, gchunks, gpre[kMaxGuestTypes + 1];
   double lrc_term[kBatchMaxTab];
-  // multi-jump (gcmc.f:1557-1785) across the two loop trips of one move: stage 1 while the
-  // first jump is evaluated and committed, 2 for the second jump; the first molecule's choice
-  // and old sites, its energy change, the energy before the move and the commit action
-  // (1: park S(k) in the chain's global copy, then commit; 2: restore S(k) and the first molecule)
-  int mj_stage, mj_first, mj_lo, mj_action;
+  // multi-jump (gcmc.f:1557-1785) across the two loop trips of one move: the first molecule's
+  // choice and old sites, and (the bookkeeping warp's) its energy change and the energy before
+  int mj_first, mj_lo;
   double mj_estep, mj_energy0;
   double mj_old[3 * kBatchMaxSites];
+};
+
+// What the acceptance test and the commit read.  Two copies in turn: the next move's set-up writes the
+// other one while slower warps still commit this one.
+struct MoveCtl {
+  int mtype, g, ns, nmols, randchoice, need_lrc;
+  int lo, seg_end;  // the moved molecule's first site, the end of its species' segment
+  int mj_stage;     // multi-jump: 1 while the first jump is evaluated and kept, 2 for the second
+  double rande;     // the draw the acceptance test takes if it draws
+  double pref;      // the acceptance test's factor of exp(-beta dE) (insert, delete)
+  int free_delete;  // no pressure: deletions are accepted
+  double lrc, elrc; // tail correction with the trial's counts, and of the state before it
+  double mj_estep;
+};
+
+// A decided move, kept for its bookkeeping (which runs beside the next move's set-up).
+struct MoveDone {
+  int mtype, g, randchoice, accepted, mj_stage, mv;
+  double ewld1, ewld2, ewld3, vdw, delrc, estep, rande;
 };
 
 // A CTA's shared memory: the chain's control block, the move in progress and the system's constants,
@@ -50,6 +71,9 @@ struct BatchSmem {
   ChainDev C;
   MoveSmem M;
   SysConst Y;
+  MoveCtl ctl[2];
+  MoveDone done;
+  int st_nmol[kMaxGuestTypes];  // the bookkeeping warp's own copy of the molecule counts
   double red[3 * 16];  // per warp {sum akk d|S|^2, ewld2, vdw}
   int prow[(kBatchMaxTypes + 1) * (kBatchMaxTypes + 1)];
 };
@@ -80,42 +104,56 @@ __device__ __forceinline__ BatchArrays batch_arrays(int kmax_smem) {
   return A;
 }
 
-// duni (gcmc.f:2712-2805) with ir, jr and c held in registers across a run of draws; the
-// arithmetic is duni_next's, draw for draw.
-struct DuniLocal {
-  float* u;
-  float c;
-  int ir, jr;
-  __device__ explicit DuniLocal(Duni& d) : u(d.u), c(d.c), ir(d.ir), jr(d.jr) {}
-  __device__ void store(Duni& d) const {
-    d.c = c;
-    d.ir = ir;
-    d.jr = jr;
-  }
-  __device__ double next() {
-    const float cd = 7654321.0f / 16777216.0f, cm = 16777213.0f / 16777216.0f;
-    float uni = u[ir - 1] - u[jr - 1];
+// The next 32 draws of duni (gcmc.f:2712-2805), one per lane.  The lagged Fibonacci part reads entries
+// 33 and 97 draws back, so 32 draws do not depend on one another, and c steps through multiples of
+// 2^-24 below cm, so lane i reaches its c in exact integer arithmetic; every draw equals duni's.
+// Serially a draw is a chain of two dependent table reads, four additions and their tests (a move takes
+// 2-11 of them, ~1.7k SM cycles); here all are ready after one such chain.
+struct DrawWarp {
+  float fresh, value, c;  // this lane's new table entry, its draw and c after it
+  int slot, used;
+
+  __device__ __forceinline__ void generate(const Duni& d, int lane) {
+    constexpr int kCm = 16777213, kCd = 7654321;
+    int i = d.ir - lane, j = d.jr - lane;
+    if (i < 1) i += 97;
+    if (j < 1) j += 97;
+    slot = i - 1;
+    float uni = d.u[i - 1] - d.u[j - 1];
     if (uni < 0.0f) uni = uni + 1.0f;
-    u[ir - 1] = uni;
-    ir = ir - 1;
-    if (ir == 0) ir = 97;
-    jr = jr - 1;
-    if (jr == 0) jr = 97;
-    c = c - cd;
-    if (c < 0.0f) c = c + cm;
+    fresh = uni;
+    const int ci = ((int)(d.c * 16777216.0f) + (lane + 1) * (kCm - kCd)) % kCm;
+    c = (float)ci * (1.0f / 16777216.0f);
     uni = uni - c;
     if (uni < 0.0f) uni = uni + 1.0f;
-    return (double)uni;
+    value = uni;
+    used = 0;
+  }
+  // Draw i of the 32 (every lane).
+  __device__ __forceinline__ double at(int i) const { return (double)__shfl_sync(0xffffffffu, value, i); }
+  // The state after the draws taken so far.
+  __device__ __forceinline__ void commit(Duni& d, int lane) {
+    if (used == 0) return;
+    const float cl = __shfl_sync(0xffffffffu, c, used - 1);
+    if (lane < used) d.u[slot] = fresh;
+    if (lane == 0) {
+      int i = d.ir - used, j = d.jr - used;
+      d.ir = i < 1 ? i + 97 : i;
+      d.jr = j < 1 ? j + 97 : j;
+      d.c = cl;
+    }
+    __syncwarp();
   }
 };
 
-// Thread 0: bookkeeping of gcmc.f:594-736 (production / termination every 400 moves),
-// random choices and the trial sites.
-// Thread 0, every 400 moves (gcmc.f:594-736): the end of production, the switch to production
-// and the pressure equilibration; a rare path, kept out of line.
-__device__ __noinline__ void check400(ChainDev& C, const SysConst& Y) {
+// Every 400 moves (gcmc.f:594-736): the end of production, the switch to production and the pressure
+// equilibration; a rare path, kept out of line.
+__device__ __noinline__ void check400() {
+  BatchSmem& B = batch_smem();
+  ChainDev& C = B.C;
+  const SysConst& Y = B.Y;
   int totalguests = 0;
-  for (int g = 0; g < Y.nspecies; g++) totalguests += C.nmol[g];
+  for (int g = 0; g < Y.nspecies; g++) totalguests += B.st_nmol[g];
   if (C.production) {
     if (C.mcsteps < 0) {
       for (int t = 4; t > 0; t--) C.tick[t] = C.tick[t - 1];
@@ -150,203 +188,175 @@ __device__ __noinline__ void check400(ChainDev& C, const SysConst& Y) {
   }
 }
 
-// Thread 0: energy assembly of the move (gcmc.f:946, 1112, 1328).  v = {sum akk*d|S|^2,
-// ewld2, vdw} as reduced by the block.
-__device__ __forceinline__ void assemble(const SysConst& Y, MoveSmem& M, const double* v) {
-  const SpeciesConst& P = Y.sp[M.g];
-  M.ewld1 = Y.S.recip_pref * v[0];
-  M.ewld2 = v[1];
-  M.vdw = v[2];
-  M.ewld3 = 0.0;
-  if (M.mtype == kInsert) {
-    M.ewld1 = M.ewld1 + P.engsic;
-    M.ewld3 = P.ewald3en;
-    M.estep = (M.ewld1 + v[1] + M.ewld3 + v[2] + M.delrc) / Y.engunit;
-  } else if (M.mtype == kDelete) {
-    M.ewld1 = M.ewld1 - P.engsic;
-    M.ewld3 = P.ewald3en;
-    M.estep = (M.ewld1 - v[1] - M.ewld3 - v[2] + M.delrc) / Y.engunit;
-  } else {
-    M.estep = (M.ewld1 + v[1] + v[2]) / Y.engunit;
-  }
+__device__ __noinline__ void insertion_sample(int i, double estep) {
+  ChainDev& C = batch_smem().C;
+  window_insertion(C.win, i, estep, C.temp, C.accept_ins, C.stats[i]);
 }
 
-// Thread 0: acceptance (energy_eval, utility_pack.f:3049-3095, with the displacement
-// shortcut of gcmc.f:1330-1338).  Random numbers are drawn exactly where the reference draws them.
-__device__ __forceinline__ void decide(ChainDev& C, const SysConst& Y, MoveSmem& M) {
-  const int g = M.g, mtype = M.mtype, nmols = C.nmol[g];
-  double e = M.estep;
-  if (mtype == kNoop) {  // nothing to accept or reject; no draw
-    M.accepted = 0;
-    return;
-  }
-  if (mtype == kMultiJump) {
-    if (M.mj_stage == 1) {  // the first jump is kept for now
-      M.accepted = 1;
-      return;
+__device__ __noinline__ void close_window() {
+  BatchSmem& B = batch_smem();
+  ChainDev& C = B.C;
+  window_close(C.win, B.Y.nspecies, C.nwind, C.temp, [&C](int i) { return (const double*)C.stats[i]; });
+}
+
+// One production move's averages (gcmc.f:1814-1928) by the bookkeeping warp: the five rolling averages and
+// the five window means of a species take a lane each (their divisions, one after another, were a
+// third of the bookkeeping); lane 0 stores the samples and takes the rare parts.  ins_g: species of an
+// accepted insertion (-1: none).
+__device__ __noinline__ void production_sample(int ins_g, bool counted, double estep, int lane) {
+  BatchSmem& B = batch_smem();
+  ChainDev& C = B.C;
+  const int ns = B.Y.nspecies;
+  const bool count = (C.laccsample && counted) || !C.laccsample;
+  const long long prodcount = C.prodcount + (count ? 1 : 0);
+  if (count) {
+    const double pc = (double)prodcount;
+    const int roll = C.win.rollcount + 1;
+    __syncwarp();
+    if (lane == 0) {
+      C.prodcount = prodcount;
+      C.win.rollcount = roll;
     }
-    e = M.mj_estep + e;  // one test on the summed change (gcmc.f:1730-1739)
-  }
-  if (mtype == kInsert || mtype == kDelete) {
-    M.rande = duni_next(C.rng);
-    M.rande_drawn = 1;
-    M.accepted = accept_move(e, M.rande, Y.statvolm, C.press[g], nmols, C.temp, C.beta, mtype);
-    return;
-  }
-  if (e < 0.0) {
-    M.accepted = 1;
-    return;
-  }
-  M.rande = duni_next(C.rng);
-  M.rande_drawn = 1;
-  M.accepted = accept_move(e, M.rande, Y.statvolm, C.press[g], nmols, C.temp, C.beta, kDisplace);
-}
-
-// Thread 0: counters, running energy, statistics and the trace record (gcmc.f:954-1380,
-// 1814-1860) once the move is decided.
-// Thread 0, production moves: the rolling averages, the stored samples and the averaging
-// windows of gcmc.f:1814-1928.  ins_g: species of an accepted insertion (-1: none).
-__device__ __noinline__ void production_sample(ChainDev& C, const SysConst& Y, int ins_g, bool counted,
-                                               double estep) {
-  if ((C.laccsample && counted) || !C.laccsample) {
-    C.prodcount++;
-    C.win.rollcount++;
-    const double pc = (double)C.prodcount;
-    for (int i = 0; i < Y.nspecies; i++) {
-      double dm = (double)(float)C.nmol[i], m2 = dm * dm, en = C.energy[i], e2 = en * en;
-      if (C.gasmol && C.prodcount <= kSampleCap + 1) {
-        C.gasmol[(size_t)i * kSampleCap + C.prodcount - 1] = dm;
-        C.gaseng[(size_t)i * kSampleCap + C.prodcount - 1] = en;
+#pragma unroll 1
+    for (int i = 0; i < ns; i++) {
+      const double dm = (double)(float)B.st_nmol[i], en = C.energy[i];
+      if (lane == 0 && C.gasmol && prodcount <= kSampleCap + 1) {
+        C.gasmol[(size_t)i * kSampleCap + prodcount - 1] = dm;
+        C.gaseng[(size_t)i * kSampleCap + prodcount - 1] = en;
       }
-      double* cs = C.stats[i];
-      cs[0] = cs[0] + (dm - cs[0]) / pc;
-      cs[1] = cs[1] + (en - cs[1]) / pc;
-      cs[2] = cs[2] + (en * dm - cs[2]) / pc;
-      cs[3] = cs[3] + (m2 - cs[3]) / pc;
-      cs[4] = cs[4] + (e2 - cs[4]) / pc;
-      window_sample(C.win, i, dm, en, ins_g == i, estep, C.temp, C.accept_ins, cs);
+      if (lane < 10) {
+        const bool rolling = lane < 5;
+        const int k = rolling ? lane : lane - 5;
+        const double v = k == 0 ? dm : (k == 1 ? en : (k == 2 ? en * dm : (k == 3 ? dm * dm : en * en)));
+        double* p = rolling ? &C.stats[i][k] : &C.win.avg[i][k];
+        const double old = *p;
+        const double q = (rolling ? v - old : (roll - 1) * old + v) / (rolling ? pc : (double)roll);
+        *p = rolling ? old + q : q;
+      }
+      __syncwarp();
+      if (lane == 0 && ins_g == i) insertion_sample(i, estep);
     }
   }
-  if (C.prodcount % C.nwind == 0 || !C.lgchk)
-    window_close(C.win, Y.nspecies, C.nwind, C.temp, [&C](int i) { return (const double*)C.stats[i]; });
+  __syncwarp();
+  const bool closes = prodcount <= 0x7fffffffLL ? (int)prodcount % C.nwind == 0 : prodcount % C.nwind == 0;
+  if (lane == 0 && (closes || !C.lgchk)) close_window();
 }
 
-__device__ __noinline__ void bookkeep(ChainDev& C, const SysConst& Y, MoveSmem& M, MoveRecord* rec) {
-  const int g = M.g, ns = M.ns, mtype = M.mtype;
-  const SpeciesConst& P = Y.sp[g];
-  const int nmols = C.nmol[g];
-  const bool accepted = M.accepted;
-  double estep = M.estep;
-  M.seg_end = C.seg_off[g] + nmols * ns;
-  if (mtype == kMultiJump) {
-    M.commit_lo = M.ex_lo;
-    if (M.mj_stage == 1) {
-      // the first jump stands while the second is tried (gcmc.f:1697-1715): remember where it
-      // came from; the move is counted once, when the second jump is decided
-      M.mj_estep = estep;
-      M.mj_lo = M.ex_lo;
-      for (int i = 0; i < ns; i++) {
-        M.mj_old[3 * i] = M.x[i];
-        M.mj_old[3 * i + 1] = M.y[i];
-        M.mj_old[3 * i + 2] = M.z[i];
-      }
-      M.mj_action = 1;
-      C.energy[g] = M.mj_energy0 + estep;
-      return;
-    }
-    estep = M.mj_estep + estep;
-    M.mj_stage = 0;
-    if (accepted) {
-      C.accept_jump++;
-      C.energy[g] = M.mj_energy0 + estep;
-    } else {
-      M.mj_action = 2;
-      C.energy[g] = M.mj_energy0;
-    }
-  }
-  if (mtype == kInsert) {
-    M.commit_lo = M.seg_end;
-    if (accepted) {
-      C.accept_ins++;
-      C.elrc = C.elrc + M.delrc;
-      C.nmol[g]++;
-      C.totatm += ns;
-      C.energy[g] += estep;
-    } else {
-      for (int i = 0; i < ns; i++) C.numtyp[P.type[i]]--;
-    }
-  } else if (mtype == kDelete) {
-    M.commit_lo = M.ex_lo;
-    if (accepted) {
-      C.accept_del++;
-      C.elrc = C.elrc + M.delrc;
-      C.nmol[g]--;
-      C.totatm -= ns;
-      C.energy[g] += estep;
-    } else {
-      for (int i = 0; i < ns; i++) C.numtyp[P.type[i]]++;
-    }
-  } else if (mtype != kNoop && mtype != kMultiJump) {
-    M.commit_lo = M.ex_lo;
-    if (accepted) {
-      if (mtype == kTranslate) C.accept_tran[g]++;
-      else if (mtype == kRotate) C.accept_rota++;
-      else if (mtype == kJump) C.accept_jump++;
-      else C.accept_disp[g]++;
-      C.energy[g] += estep;
-    }
-  }
+// Bookkeeping of a decided move (gcmc.f:954-1380, 1796-1928) by one warp, beside the next move's
+// set-up: running energies, the counters the set-up does not read, statistics, the trace record.
+__device__ __noinline__ void finish_move(MoveRecord* trace, int lane) {
+  BatchSmem& B = batch_smem();
+  ChainDev& C = B.C;
+  MoveSmem& M = B.M;
+  __syncwarp();  // lane 0 wrote the decided move
+  const MoveDone D = B.done;
+  const int g = D.g, mtype = D.mtype;
+  const bool accepted = D.accepted != 0;
+  double estep = D.estep;
+  const bool first_jump = mtype == kMultiJump && D.mj_stage == 1;
+  if (mtype == kMultiJump && !first_jump) estep = M.mj_estep + estep;
   // flex / swap leave the reference's `accepted` as the previous move set it
   const bool counted = mtype == kNoop ? (C.last_accepted != 0) : accepted;
-  if (mtype != kNoop) C.last_accepted = accepted;
-  if (C.production) production_sample(C, Y, mtype == kInsert && accepted ? g : -1, counted, estep);
-  else if (C.despre > 0 && ((C.laccsample && counted) || !C.laccsample)) {
+  __syncwarp();
+  if (lane == 0) {
+    if (first_jump) {
+      // the first jump stands while the second is tried (gcmc.f:1697-1715); the move is counted
+      // once, when the second jump is decided
+      M.mj_energy0 = C.energy[g];
+      M.mj_estep = estep;
+      C.energy[g] = M.mj_energy0 + estep;
+      C.jump_count++;
+    } else if (mtype == kMultiJump) {
+      if (accepted) C.accept_jump++;
+      C.energy[g] = accepted ? M.mj_energy0 + estep : M.mj_energy0;
+    } else if (mtype == kNoop) {
+    } else {
+      if (mtype == kInsert) C.ins_count++;
+      else if (mtype == kDelete) C.del_count++;
+      else if (mtype == kJump) C.jump_count++;
+      if (accepted) {
+        if (mtype == kInsert || mtype == kDelete) {
+          if (mtype == kInsert) C.accept_ins++;
+          else C.accept_del++;
+          C.elrc = C.elrc + D.delrc;
+          B.st_nmol[g] += mtype == kInsert ? 1 : -1;
+        } else if (mtype == kJump) {
+          C.accept_jump++;
+        }
+        C.energy[g] += estep;
+      }
+    }
+    if (!first_jump) {
+      if (mtype != kNoop) C.last_accepted = accepted;
+      C.last_dE = accepted ? estep : 0.0;
+      C.moves_done++;
+    }
+  }
+  __syncwarp();
+  if (first_jump) return;
+  if (C.production) {
+    production_sample(mtype == kInsert && accepted ? g : -1, counted, estep, lane);
+  } else if (lane == 0 && C.despre > 0 && ((C.laccsample && counted) || !C.laccsample)) {
     // running loading while the pressures equilibrate (gcmc.f:1796-1808)
     C.prodcount++;
-    for (int i = 0; i < Y.nspecies; i++)
-      C.stats[i][0] = C.stats[i][0] + ((double)(float)C.nmol[i] - C.stats[i][0]) / (double)C.prodcount;
+#pragma unroll 1
+    for (int i = 0; i < B.Y.nspecies; i++)
+      C.stats[i][0] = C.stats[i][0] + ((double)(float)B.st_nmol[i] - C.stats[i][0]) / (double)C.prodcount;
   }
-  C.last_dE = accepted ? estep : 0.0;
-  C.moves_done++;
-  if (rec) {
+  if (trace && lane == 0) {
+    MoveRecord* rec = trace + D.mv;
     rec->step = C.gcmccount;
     rec->iguest = g;
     rec->mtype = mtype;
-    rec->randchoice = M.randchoice;
+    rec->randchoice = D.randchoice;
     rec->accepted = counted;  // as the reference's `accepted` reads after the move
-    rec->nmols_after = C.nmol[g];
+    rec->nmols_after = B.st_nmol[g];
     rec->pad0 = 0;
     rec->pad1 = 0;
-    rec->ewld1 = M.ewld1;
-    rec->ewld2 = M.ewld2;
-    rec->ewld3 = M.ewld3;
-    rec->vdw = M.vdw;
-    rec->delrc = M.delrc;
+    rec->ewld1 = D.ewld1;
+    rec->ewld2 = D.ewld2;
+    rec->ewld3 = D.ewld3;
+    rec->vdw = D.vdw;
+    rec->delrc = D.delrc;
     rec->estep = estep;
-    rec->rande = M.rande;
+    rec->rande = D.rande;
     rec->energy_after = C.energy[g];
   }
+  __syncwarp();
 }
 
-// Tail correction (gstlrcorrect, vdw_terms.f:684-745) by one warp: lane-parallel pair terms,
-// summed by lane 0 in the reference's pair order.
-__device__ __forceinline__ void lrc_warp(const ChainDev& C, const SysConst& Y, MoveSmem& M, int lane) {
+// Tail correction (gstlrcorrect, vdw_terms.f:684-745) by one warp, with the trial's molecule added to
+// (d = 1) or taken from (-1) the counts: lane-parallel pair terms, summed by lane 0 in the reference's
+// pair order.
+__device__ __forceinline__ void lrc_warp(const BatchSmem& B, MoveSmem& M, int g, int d, double& lrc, int lane) {
+  const ChainDev& C = B.C;
+  const SysConst& Y = B.Y;
+  const SpeciesConst& P = Y.sp[g];
   const int nt = Y.ntypes, ntab = nt * (nt + 1) / 2;
   const double twopi = 2.0 * kPi, v = Y.volm;
+#pragma unroll 1
   for (int p = lane; p < ntab; p += 32) {
     int i = 1;
+#pragma unroll 1
     while (i * (i + 1) / 2 <= p) i++;
     int j = p - (i - 1) * i / 2 + 1;
-    double den =
-        twopi * ((double)C.numtyp[i] * (double)C.numtyp[j] - (double)Y.numfrz[i] * (double)Y.numfrz[j]) / (v * v);
+    int ni = C.numtyp[i], nj = C.numtyp[j];
+#pragma unroll 1
+    for (int s = 0; s < P.nsite; s++) {
+      const int t = P.type[s];
+      if (t == i) ni += d;
+      if (t == j) nj += d;
+    }
+    double den = twopi * ((double)ni * (double)nj - (double)Y.numfrz[i] * (double)Y.numfrz[j]) / (v * v);
     M.lrc_term[p] = v * den * Y.steadd[p + 1];
   }
   __syncwarp();
   if (lane == 0) {
     double e = 0.0;
     if (Y.lrc_on)
+#pragma unroll 4
       for (int p = 0; p < ntab; p++) e = e + M.lrc_term[p];
-    M.delrc = e - C.elrc;
+    lrc = e;
   }
 }
 
@@ -357,165 +367,156 @@ __device__ __forceinline__ long long global_ns() {
   return (long long)t;
 }
 
-// Warp 0: phase tables of the trial sites (ewald.f:95-137).  The first axis carries the site's
+// One warp: phase tables of the trial sites (ewald.f:95-137).  The first axis carries the site's
 // charge, negative for a site that leaves, so that the reciprocal loop only multiplies and adds.
-__device__ __forceinline__ void build_phases(const SysConst& Y, const MoveSmem& M, double2* tab, int stride, int lane) {
-  const DevSystem& S = Y.S;
+__device__ __forceinline__ void build_phases(const BatchSmem& B, double2* tab, int stride, int lane) {
+  const MoveSmem& M = B.M;
+  const DevSystem& S = B.Y.S;
   const int nold = M.nold, nsite = nold + M.nnew, k1 = S.kmax[0], k2 = S.kmax[1];
+  const SpeciesConst& P = B.Y.sp[M.g];
+#pragma unroll 1
   for (int w = lane; w < nsite * 3; w += 32) {
     int st = w / 3, ax = w % 3;
     double f[3];
     frac_coords(S.cell, M.x[st], M.y[st], M.z[st], f);
     int off = st * stride + (ax == 0 ? 0 : (ax == 1 ? k1 + 1 : k1 + k2 + 2));
-    const double q = ax ? 1.0 : (st < nold ? -Y.sp[M.g].q[st] : Y.sp[M.g].q[st - nold]);
+    const double q = ax ? 1.0 : (st < nold ? -P.q[st] : P.q[st - nold]);
     axis_phases(f[ax], S.kmax[ax], tab + off, q);
   }
 }
 
-// Lane 0 of warp 0: the serial part of a move's set-up (gcmc.f:594-847): the move count and
-// the 400-move checks, species and move choice, step-size adaptation, the counters, and every
-// random number of the trial in the reference's order (utility_pack.f:2545-3000), which
-// select_move leaves in M.r for the warp to build the trial sites from.
-template <bool kProf>
-__device__ __noinline__ void select_move(ChainDev& C, const SysConst& Y, MoveSmem& M) {
-  if (kProf) C.prof[7] -= clock64();
-  M.mj_action = 0;
-  const bool second = M.mj_stage == 1;  // the second jump of a multi-jump: no count or selection
-  if (!second) {
-    M.mj_first = 0;  // a new move: no molecule to avoid
-    C.gcmccount++;
-    if (C.gcmccount % 400 == 0) check400(C, Y);
-  }
-  DuniLocal R(C.rng);  // written back before every return
-  int g = M.g, mtype = kMultiJump;
-  if (second) {
-    M.mj_stage = 2;
-  } else {
-  const int ng = Y.nspecies;
-  g = 0;
-  if (ng > 1) g = (int)floor(R.next() * ng);
-  double randmov = R.next();
-  const double* c = C.mvcum[g];
-  if (randmov < c[0]) mtype = kInsert;
-  else if (randmov < c[1]) mtype = kDelete;
-  else if (randmov < c[2]) mtype = kDisplace;
-  else if (randmov < c[3]) mtype = kJump;
-  else if (randmov < c[5]) mtype = kNoop;  // flex, swap (gcmc.f:1789-1795)
-  else if (randmov < c[6]) mtype = kTranslate;
-  else if (randmov < c[7]) mtype = kRotate;
-  else if (randmov < c[8]) mtype = kMultiJump;
-  else mtype = kDisplace;
-  const int nmols = C.nmol[g];
-  // step-size adaptation (gcmc.f:794-834)
-  if (nmols >= 1 && C.disp_count[g] >= 1) {
-    if (C.disp_count[g] % 100 == 0) {
-      if ((C.accept_disp[g] / (double)C.disp_count[g]) > C.disp_ratio[g]) C.delrdisp[g] = C.delrdisp[g] * 1.05;
+// Warp 0: the serial part of a move's set-up (gcmc.f:753-847): species and move choice, step-size
+// adaptation, the counters it reads, and every random number of the trial in the reference's order
+// (utility_pack.f:2545-3000), left in r for the warp to build the trial sites from.  Every lane
+// takes the same branches and lane 0 writes.  `skip`: the last move's acceptance test took a draw.
+// Past the 32nd draw (a multi-jump that keeps drawing its first molecule): the state moves on.
+__device__ __noinline__ DrawWarp refill_draws(DrawWarp R, int lane) {
+  Duni& d = batch_smem().C.rng;
+  R.commit(d, lane);
+  R.generate(d, lane);
+  return R;
+}
+
+// Step-size adaptation (gcmc.f:794-834), every 50 or 100 attempts; out of line so that the set-up's code,
+// run once a move, stays small (its instruction fetches are most of its time).
+__device__ __noinline__ void adapt_steps(int g) {
+  ChainDev& C = batch_smem().C;
+  const int dc = C.disp_count[g], tc = C.tran_count[g], rc = C.rota_count;
+  if (dc >= 1 && dc % 50 == 0) {
+    const bool over = (C.accept_disp[g] / (double)dc) > C.disp_ratio[g];
+    if (dc % 100 == 0) {
+      if (over) C.delrdisp[g] = C.delrdisp[g] * 1.05;
       else if (C.delrdisp[g] > kDelrMin) C.delrdisp[g] = C.delrdisp[g] * 0.95;
-    } else if (C.disp_count[g] % 50 == 0) {
-      if ((C.accept_disp[g] / (double)C.disp_count[g]) > C.disp_ratio[g]) C.rotangle = C.rotangle * 1.05;
+    } else {
+      if (over) C.rotangle = C.rotangle * 1.05;
       else if (C.rotangle > kMinAngle) C.rotangle = C.rotangle * 0.95;
     }
   }
-  if (nmols >= 1 && C.tran_count[g] >= 1 && C.tran_count[g] % 100 == 0) {
-    if ((C.accept_tran[g] / (double)C.tran_count[g]) > C.tran_ratio[g]) C.tran_delr[g] = C.tran_delr[g] * 1.05;
+  if (tc >= 1 && tc % 100 == 0) {
+    if ((C.accept_tran[g] / (double)tc) > C.tran_ratio[g]) C.tran_delr[g] = C.tran_delr[g] * 1.05;
     else if (C.tran_delr[g] > kDelrMin) C.tran_delr[g] = C.tran_delr[g] * 0.95;
   }
-  if (nmols >= 1 && C.rota_count >= 1 && C.rota_count % 100 == 0) {
-    if ((C.accept_rota / (double)C.rota_count) > C.rota_ratio) C.rota_rotangle = C.rota_rotangle * 1.05;
+  if (rc >= 1 && rc % 100 == 0) {
+    if ((C.accept_rota / (double)rc) > C.rota_ratio) C.rota_rotangle = C.rota_rotangle * 1.05;
     else if (C.rota_rotangle > kMinAngle) C.rota_rotangle = C.rota_rotangle * 0.95;
   }
-  if (nmols == 0 || (nmols == 1 && mtype == kMultiJump)) mtype = kInsert;  // gcmc.f:837-847
-  if (mtype == kMultiJump) {
-    C.jump_count++;
-    M.mj_stage = 1;
-    M.mj_first = 0;
-    M.mj_energy0 = C.energy[g];
-  }
-  }
-  const SpeciesConst& P = Y.sp[g];
-  const int ns = P.nsite, nmols = C.nmol[g];
-  if (kProf) C.prof[7] += clock64();  // minus the stamp taken at entry: selection + adaptation
-  M.mtype = mtype;
-  M.g = g;
-  M.ns = ns;
-  M.mol = -1;
-  M.randchoice = 0;
-  M.ex_lo = M.ex_hi = -1;
-  M.nold = M.nnew = 0;
-  M.delrc = 0.0;
-  M.rande = -1.0;
-  M.need_lrc = 0;
-  M.rande_drawn = 0;
-  double* r = M.r;
-  if (mtype == kInsert) {
-    C.ins_count++;
-    if ((C.totatm - C.framatm) + ns >= C.maxguest || (nmols + 1) * ns > C.seg_cap[g]) {
-      C.status = 75;
-      R.store(C.rng);
-      return;
+}
+
+__device__ __noinline__ void select_move(int par, int skip, bool second, int lane) {
+  BatchSmem& B = batch_smem();
+  ChainDev& C = B.C;
+  const SysConst& Y = B.Y;
+  MoveSmem& M = B.M;
+  MoveCtl& T = B.ctl[par];
+  DrawWarp R;
+  R.generate(C.rng, lane);
+  R.used = skip;
+  int g = 0, mtype = kMultiJump, mj_stage = 2, mj_first = 0;
+  if (second) {  // the second jump of a multi-jump: no count or selection
+    g = M.g;
+    mj_first = M.mj_first;
+  } else {
+    const int ng = Y.nspecies;
+    if (ng > 1) g = (int)(R.at(R.used++) * ng);
+    // the first cumulative frequency above the draw: insert, delete, displace, jump, flex and swap
+    // (gcmc.f:1789-1795), translate, rotate, multi-jump; none: displace
+    const double randmov = R.at(R.used++);
+    const unsigned above = __ballot_sync(0xffffffffu, lane < 9 && randmov < C.mvcum[g][lane < 9 ? lane : 0]);
+    constexpr unsigned long long kTypes = 0x854776321ULL;
+    static_assert(kInsert == 1 && kDelete == 2 && kDisplace == 3 && kTranslate == 4 && kRotate == 5 && kJump == 6 &&
+                      kNoop == 7 && kMultiJump == 8, "one digit of kTypes each");
+    mtype = above ? (int)(kTypes >> (4 * (__ffs(above) - 1))) & 15 : (int)kDisplace;
+    const int nmols = C.nmol[g];
+    const unsigned dc = C.disp_count[g], tc = C.tran_count[g], rc = C.rota_count;
+    if (nmols >= 1 && ((dc && dc % 50u == 0) || (tc && tc % 100u == 0) || (rc && rc % 100u == 0))) {
+      if (lane == 0) adapt_steps(g);
+      __syncwarp();
     }
-    for (int i = 0; i < 7; i++) r[i] = R.next();
-    M.nnew = ns;
-    for (int i = 0; i < ns; i++) C.numtyp[P.type[i]]++;
-    M.need_lrc = 1;
-  } else if (mtype == kDelete) {
-    C.del_count++;
-    int randchoice = (int)floor(R.next() * nmols) + 1;
-    M.randchoice = randchoice;
-    M.mol = randchoice - 1;
-    M.ex_lo = C.seg_off[g] + M.mol * ns;
-    M.ex_hi = M.ex_lo + ns;
-    M.nold = ns;
-    for (int i = 0; i < ns; i++) C.numtyp[P.type[i]]--;
-    M.need_lrc = 1;
-  } else if (mtype == kJump || mtype == kMultiJump) {
+    if (nmols == 0 || (nmols == 1 && mtype == kMultiJump)) mtype = kInsert;  // gcmc.f:837-847
+    mj_stage = mtype == kMultiJump ? 1 : 0;
+  }
+  const int ns = Y.sp[g].nsite, nmols = C.nmol[g], seg = C.seg_off[g];
+  const bool jump = mtype == kJump || mtype == kMultiJump, need_lrc = mtype == kInsert || mtype == kDelete;
+  const bool full = mtype == kInsert && ((C.totatm - C.framatm) + ns >= C.maxguest || (nmols + 1) * ns > C.seg_cap[g]);
+  int randchoice = 0;
+  if (jump) {
     // long jump (gcmc.f:1389-1547): the choice first, then the seven draws of random_jump; the
     // second jump of a multi-jump draws until it hits a molecule other than the first
-    if (mtype == kJump) C.jump_count++;
-    int randchoice;
     do {
-      randchoice = (int)floor(R.next() * nmols) + 1;
-    } while (randchoice == M.mj_first);
-    if (mtype == kMultiJump && M.mj_stage == 1) M.mj_first = randchoice;
-    M.randchoice = randchoice;
-    M.mol = randchoice - 1;
-    M.ex_lo = C.seg_off[g] + M.mol * ns;
-    M.ex_hi = M.ex_lo + ns;
-    for (int i = 0; i < 7; i++) r[i] = R.next();
-    M.nold = ns;
-    M.nnew = ns;
-  } else if (mtype == kNoop) {
-    // nothing moves; no sites, no draws beyond the move choice
-  } else {
+      if (R.used == 32) R = refill_draws(R, lane);
+      randchoice = (int)(R.at(R.used++) * nmols) + 1;
+    } while (randchoice == mj_first);
+    if (mj_stage == 1) mj_first = randchoice;
+    if (R.used > 24) R = refill_draws(R, lane);
+  }
+  // r[0..6], lane i's r[i]: a translation draws the first three, a rotation the last four
+  const int lo = mtype == kRotate ? 3 : 0;
+  const int nr = mtype == kDelete || mtype == kNoop || full ? 0 : (mtype == kTranslate ? 3 : 7 - lo);
+  const double drawn = R.at((R.used + lane - lo) & 31);
+  const double r = lane >= lo && lane < lo + nr ? drawn : (mtype == kRotate ? 0.5 : 0.0);
+  R.used += nr;
+  if (mtype == kDelete || mtype == kDisplace || mtype == kTranslate || mtype == kRotate)
+    randchoice = (int)(R.at(R.used++) * nmols) + 1;
+  const double rande = R.at(R.used);  // the draw the acceptance test would take (at most the 32nd)
+  R.commit(C.rng, lane);
+  if (lane < 7) M.r[lane] = r;
+  if (lane == 0) {
+    if (full) C.status = 75;
+    double dis_delr = 0.0, dis_rot = 0.0;
     if (mtype == kTranslate) {
       C.tran_count[g]++;
-      r[0] = R.next();
-      r[1] = R.next();
-      r[2] = R.next();
-      r[3] = r[4] = r[5] = r[6] = 0.0;
-      M.dis_delr = C.tran_delr[g];
-      M.dis_rot = 0.0;
+      dis_delr = C.tran_delr[g];
     } else if (mtype == kRotate) {
       C.rota_count++;
-      r[0] = r[1] = r[2] = 0.5;
-      for (int i = 3; i < 7; i++) r[i] = R.next();
-      M.dis_delr = 0.0;
-      M.dis_rot = C.rota_rotangle;
-    } else {
+      dis_rot = C.rota_rotangle;
+    } else if (mtype == kDisplace) {
       C.disp_count[g]++;
-      for (int i = 0; i < 7; i++) r[i] = R.next();
-      M.dis_delr = C.delrdisp[g];
-      M.dis_rot = C.rotangle;
+      dis_delr = C.delrdisp[g];
+      dis_rot = C.rotangle;
     }
-    int randchoice = (int)floor(R.next() * nmols) + 1;
-    M.randchoice = randchoice;
-    M.mol = randchoice - 1;
-    M.ex_lo = C.seg_off[g] + M.mol * ns;
-    M.ex_hi = M.ex_lo + ns;
-    M.nold = ns;
-    M.nnew = ns;
+    M.dis_delr = dis_delr;
+    M.dis_rot = dis_rot;
+    const int first = randchoice > 0 ? seg + (randchoice - 1) * ns : -1;
+    M.mtype = mtype;
+    M.g = g;
+    M.nold = mtype == kInsert || mtype == kNoop ? 0 : ns;
+    M.nnew = mtype == kDelete || mtype == kNoop || full ? 0 : ns;
+    M.ns = ns;
+    M.ex_lo = first;
+    M.ex_hi = first < 0 ? -1 : first + ns;
+    M.mj_first = mj_first;
+    T.mtype = mtype;
+    T.g = g;
+    T.ns = ns;
+    T.nmols = nmols;
+    T.randchoice = randchoice;
+    T.need_lrc = need_lrc;
+    T.seg_end = seg + nmols * ns;
+    T.lo = mtype == kInsert ? seg + nmols * ns : first;
+    T.mj_stage = mj_stage;
+    T.rande = rande;
   }
-  R.store(C.rng);
+  __syncwarp();
 }
 
 // ------------------------------------------------------------------ the trial sites, one lane each
@@ -525,6 +526,7 @@ __device__ __noinline__ void select_move(ChainDev& C, const SysConst& Y, MoveSme
 // same centre.
 __device__ __forceinline__ void com_lanes(const double* mass, int n, double x, double y, double z, double* c) {
   double w = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
+#pragma unroll 1
   for (int j = 0; j < n; j++) {
     const double xj = __shfl_sync(0xffffffffu, x, j), yj = __shfl_sync(0xffffffffu, y, j),
                  zj = __shfl_sync(0xffffffffu, z, j);
@@ -554,141 +556,127 @@ __device__ __forceinline__ void rotate_site(const double q[4], double& x, double
   z = tz;
 }
 
+// random_jump's frame (utility_pack.f:2766-2813): the site about the mass centre once it has moved to
+// cm, and that centre.
+__device__ __noinline__ void jump_frame(const double* mass, int ns, double& x, double& y, double& z, double* cm) {
+  double c[3];
+  com_lanes(mass, ns, x, y, z, c);
+  const double xd = cm[0] - c[0], yd = cm[1] - c[1], zd = cm[2] - c[2];
+  x = xd + x;
+  y = yd + y;
+  z = zd + z;
+  com_lanes(mass, ns, x, y, z, cm);
+  x = x - cm[0];
+  y = y - cm[1];
+  z = z - cm[2];
+}
+
 // Warp 0, after select_move: the trial sites (old sites read from the chain, new ones built by
-// random_ins / random_disp + random_rot / random_jump), their charges and types, their voxel lists
-// and the real-space work list, then their phase tables (ewald.f:95-137).
-template <bool kProf>
-__device__ __noinline__ void build_trial(ChainDev& C, const SysConst& Y, const DevSystem& S, MoveSmem& M, double2* tab,
-                                         int stride, int lane) {
-  if (kProf && lane == 0) C.prof[8] -= clock64();
-  const int mtype = M.mtype, ns = M.ns, nold = M.nold, nnew = M.nnew, nseg = Y.nspecies;
+// random_ins / random_disp + random_rot / random_jump), their charges and types -- from which warp 2
+// builds the phase tables (named barrier 2) -- then their voxel lists and the real-space work list.
+__device__ __noinline__ void build_trial(int lane) {
+  BatchSmem& B = batch_smem();
+  ChainDev& C = B.C;
+  MoveSmem& M = B.M;
+  const SysConst& Y = B.Y;
+  const DevSystem& S = Y.S;
+  const int mtype = M.mtype, ns = M.ns, nold = M.nold, nnew = M.nnew;
   const SpeciesConst& P = Y.sp[M.g];
   const bool mine = lane < ns;
-  double ox = 0.0, oy = 0.0, oz = 0.0, nx = 0.0, ny = 0.0, nz = 0.0;
-  int vb_old = 0, vl_old = 0;
   if (nold && mine) {
     const double4 a = C.gsite[M.ex_lo + lane];
-    ox = a.x;
-    oy = a.y;
-    oz = a.z;
-    // the old site's voxel list, looked up while the trial geometry is computed
-    const int v = voxel_of(S, ox, oy, oz);
-    vb_old = S.vox_off[v];
-    vl_old = S.vox_off[v + 1] - vb_old;
-  }
-  const double* r = M.r;
-  const double* h = S.cell.h;
-  if (mtype == kInsert) {
-    // random_ins (utility_pack.f:2545-2650): template rotated, centred at fractional (r0, r1, r2)
-    const double xc = r[0] * h[0] + r[1] * h[3] + r[2] * h[6];
-    const double yc = r[0] * h[1] + r[1] * h[4] + r[2] * h[7];
-    const double zc = r[0] * h[2] + r[1] * h[5] + r[2] * h[8];
-    double q[4];
-    axis_angle_quat(r[3] * 2.0 * kPi, r[4], r[5], r[6], q);
-    if (mine) {
-      nx = P.tx[lane];
-      ny = P.ty[lane];
-      nz = P.tz[lane];
-      rotate_site(q, nx, ny, nz);
-      nx = nx + xc;
-      ny = ny + yc;
-      nz = nz + zc;
-    }
-  } else if (mtype == kJump || mtype == kMultiJump) {
-    // random_jump: the mass centre moved to fractional (r0, r1, r2), a new orientation about it
-    double xd = r[0] * h[0] + r[1] * h[3] + r[2] * h[6];
-    double yd = r[0] * h[1] + r[1] * h[4] + r[2] * h[7];
-    double zd = r[0] * h[2] + r[1] * h[5] + r[2] * h[8];
-    double cm[3];
-    com_lanes(P.mass, ns, ox, oy, oz, cm);
-    xd = xd - cm[0];
-    yd = yd - cm[1];
-    zd = zd - cm[2];
-    nx = xd + ox;
-    ny = yd + oy;
-    nz = zd + oz;
-    com_lanes(P.mass, ns, nx, ny, nz, cm);
-    nx = nx - cm[0];
-    ny = ny - cm[1];
-    nz = nz - cm[2];
-    double q[4];
-    axis_angle_quat(r[3] * (8.0 * atan(1.0)), r[4], r[5], r[6], q);
-    rotate_site(q, nx, ny, nz);
-    nx = nx + cm[0];
-    ny = ny + cm[1];
-    nz = nz + cm[2];
-  } else if (mtype == kDisplace || mtype == kTranslate || mtype == kRotate) {
-    // random_disp + random_rot (utility_pack.f:2679-2763, 2929-3000)
-    const double half = M.dis_delr * 0.5;
-    const double dx = (2.0 * r[0] - 1.0) * half, dy = (2.0 * r[1] - 1.0) * half, dz = (2.0 * r[2] - 1.0) * half;
-    nx = dx + ox;
-    ny = dy + oy;
-    nz = dz + oz;
-    double cm[3];
-    com_lanes(P.mass, ns, nx, ny, nz, cm);
-    const double* rh = S.cell.rh;
-    double fx = rh[0] * cm[0] + rh[3] * cm[1] + rh[6] * cm[2];
-    double fy = rh[1] * cm[0] + rh[4] * cm[1] + rh[7] * cm[2];
-    double fz = rh[2] * cm[0] + rh[5] * cm[1] + rh[8] * cm[2];
-    fx = fx - floor(fx);
-    fy = fy - floor(fy);
-    fz = fz - floor(fz);
-    const double wx = h[0] * fx + h[3] * fy + h[6] * fz;
-    const double wy = h[1] * fx + h[4] * fy + h[7] * fz;
-    const double wz = h[2] * fx + h[5] * fy + h[8] * fz;
-    const double shx = wx - cm[0], shy = wy - cm[1], shz = wz - cm[2];
-    nx = nx + shx - wx;
-    ny = ny + shy - wy;
-    nz = nz + shz - wz;
-    double q[4];
-    axis_angle_quat(r[3] * M.dis_rot, r[4], r[5], r[6], q);
-    rotate_site(q, nx, ny, nz);
-    nx = nx + wx;
-    ny = ny + wy;
-    nz = nz + wz;
-  }
-  // the work list: each trial site's voxel list, then every guest site
-  if (mine && nold) {
-    M.x[lane] = ox;
-    M.y[lane] = oy;
-    M.z[lane] = oz;
+    M.x[lane] = a.x;
+    M.y[lane] = a.y;
+    M.z[lane] = a.z;
     M.cq[lane] = (nnew ? -P.q[lane] : P.q[lane]) * kR4pie0;
-    M.type[lane] = P.type[lane];
-    M.vb[lane] = vb_old;
-    M.vl[lane] = vl_old;
+    M.type[lane] = P.type[lane] * (S.ntypes + 1);
   }
-  if (mine && nnew) {
-    const int st = nold + lane;
-    M.x[st] = nx;
-    M.y[st] = ny;
-    M.z[st] = nz;
-    M.cq[st] = P.q[lane] * kR4pie0;
-    M.type[st] = P.type[lane];
-    const int v = voxel_of(S, nx, ny, nz);
-    M.vb[st] = S.vox_off[v];
-    M.vl[st] = S.vox_off[v + 1] - S.vox_off[v];
+  if (nnew) {
+    // one code path for every move type, so that it stays small: the site about the centre of
+    // rotation (vx, vy, vz), the centre, the angle
+    const double* r = M.r;
+    const double* h = S.cell.h;
+    double vx = 0.0, vy = 0.0, vz = 0.0, cm[3], turn = 2.0 * kPi;
+    if (mine) {
+      vx = nold ? M.x[lane] : P.tx[lane];
+      vy = nold ? M.y[lane] : P.ty[lane];
+      vz = nold ? M.z[lane] : P.tz[lane];
+    }
+    if (!nold || mtype == kJump || mtype == kMultiJump) {
+      // random_ins (utility_pack.f:2545-2650): template rotated, centred at fractional (r0, r1, r2)
+      cm[0] = r[0] * h[0] + r[1] * h[3] + r[2] * h[6];
+      cm[1] = r[0] * h[1] + r[1] * h[4] + r[2] * h[7];
+      cm[2] = r[0] * h[2] + r[1] * h[5] + r[2] * h[8];
+      // random_jump: the mass centre moved there, a new orientation about it
+      if (nold) jump_frame(P.mass, ns, vx, vy, vz, cm);
+    } else {
+      // random_disp + random_rot (utility_pack.f:2679-2763, 2929-3000)
+      const double half = M.dis_delr * 0.5;
+      const double dx = (2.0 * r[0] - 1.0) * half, dy = (2.0 * r[1] - 1.0) * half, dz = (2.0 * r[2] - 1.0) * half;
+      vx = dx + vx;
+      vy = dy + vy;
+      vz = dz + vz;
+      com_lanes(P.mass, ns, vx, vy, vz, cm);
+      const double* rh = S.cell.rh;
+      double fx = rh[0] * cm[0] + rh[3] * cm[1] + rh[6] * cm[2];
+      double fy = rh[1] * cm[0] + rh[4] * cm[1] + rh[7] * cm[2];
+      double fz = rh[2] * cm[0] + rh[5] * cm[1] + rh[8] * cm[2];
+      fx = fx - floor(fx);
+      fy = fy - floor(fy);
+      fz = fz - floor(fz);
+      const double wx = h[0] * fx + h[3] * fy + h[6] * fz;
+      const double wy = h[1] * fx + h[4] * fy + h[7] * fz;
+      const double wz = h[2] * fx + h[5] * fy + h[8] * fz;
+      const double shx = wx - cm[0], shy = wy - cm[1], shz = wz - cm[2];
+      vx = vx + shx - wx;
+      vy = vy + shy - wy;
+      vz = vz + shz - wz;
+      cm[0] = wx;
+      cm[1] = wy;
+      cm[2] = wz;
+      turn = M.dis_rot;
+    }
+    double q[4];
+    axis_angle_quat(r[3] * turn, r[4], r[5], r[6], q);
+    rotate_site(q, vx, vy, vz);
+    if (mine) {
+      const int st = nold + lane;
+      M.x[st] = vx + cm[0];
+      M.y[st] = vy + cm[1];
+      M.z[st] = vz + cm[2];
+      M.cq[st] = P.q[lane] * kR4pie0;
+      M.type[st] = P.type[lane] * (S.ntypes + 1);
+    }
   }
   __syncwarp();
-  build_phases(Y, M, tab, stride, lane);
-  // work-list prefix over the sites: each site's voxel list plus every guest site, in chunks of 32
-  // (warp scan)
+  asm volatile("bar.arrive 2, 64;" ::: "memory");
+  // the work list (warp scan over the voxel lists' chunks; the guest lists have one length)
+  const int nsite = nold + nnew;
+  int b = 0, len = 0;
+  if (lane < nsite) {
+    const int v = voxel_of(S, M.x[lane], M.y[lane], M.z[lane]);
+    b = S.vox_off[v];
+    len = S.vox_off[v + 1] - b;
+  }
   int gt = 0;
-  for (int g = 0; g < nseg; g++) gt += C.nmol[g] * Y.sp[g].nsite;
-  int w = lane < nold + nnew ? (M.vl[lane] + gt + 31) >> 5 : 0;
+  if (lane == 0) M.gpre[0] = 0;
+#pragma unroll 1
+  for (int g = 0; g < Y.nspecies; g++) {
+    gt += C.nmol[g] * Y.sp[g].nsite;
+    if (lane == 0) M.gpre[g + 1] = gt;
+  }
+  const int mine_chunks = (len + 31) >> 5, gchunks = (gt + 31) >> 5;
+  int w = mine_chunks;
+#pragma unroll 1
   for (int o = 1; o < 32; o <<= 1) {
     const int u = __shfl_up_sync(0xffffffffu, w, o);
     if (lane >= o) w += u;
   }
-  if (lane < nold + nnew) M.cpre[lane + 1] = w;
+  const int fw = __shfl_sync(0xffffffffu, w, 31);
+  if (lane < nsite) M.list[lane] = make_int4(w - mine_chunks, b, len, 0);
   if (lane == 0) {
-    M.cpre[0] = 0;
-    int acc = 0;
-    M.gpre[0] = 0;
-    for (int g = 0; g < nseg; g++) {
-      acc += C.nmol[g] * Y.sp[g].nsite;
-      M.gpre[g + 1] = acc;
-    }
-    if (kProf) C.prof[8] += clock64();
+    M.nfw = fw;
+    M.gchunks = gchunks;
   }
 }
 
@@ -711,7 +699,7 @@ __device__ __forceinline__ double2 recip_term(int k, int nsite, int k1, int k2, 
   const int sm = m & 0x80000000, sn = n & 0x80000000;
   double ax = 0.0, ay = 0.0;
   const double2* t = tb;
-#pragma unroll 3
+#pragma unroll 1
   for (int st = 0; st < nsite; st++, t += stride) {
     const double2 e1 = t[l], e2 = t[o2], e3 = t[o3];
     const double y2 = flip_sign(e2.y, sm), y3 = flip_sign(e3.y, sn);
@@ -723,8 +711,12 @@ __device__ __forceinline__ double2 recip_term(int k, int nsite, int k1, int k2, 
   }
   const double2 so = Sk[k], sw = make_double2(so.x + ax, so.y + ay);
   Sn[k] = sw;
-  return make_double2(ak[k], sw.x * sw.x + sw.y * sw.y - so.x * so.x - so.y * so.y);
+  // one order of roundings: uncharged molecules leave S(k) as it is, and what rounds off here decides
+  // their moves without an energy change (real_space_residue)
+  return make_double2(ak[k], fma(-so.y, so.y, fma(-so.x, so.x, fma(sw.x, sw.x, sw.y * sw.y))));
 }
+
+constexpr double kMagic = 6755399441055744.0;  // 1.5 x 2^52: adding it rounds to an integer
 
 // How a chunk's pairs are imaged and tabulated, compiled separately so that the loop holds one form
 // (each copy costs instruction cache): orthorhombic cells (imcon 1, 2) and parallelepipeds (3) with
@@ -739,36 +731,53 @@ struct Cand {
   int type, site;
 };
 
-__device__ __forceinline__ void load_site(const double4* p, Cand& c) {
-  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(c.x), "=d"(c.y), "=d"(c.z), "=d"(c.q) : "l"(p));
-}
-
-// Chunk `chunk` of the work list: 32 candidates of one site.  `incl` is lane s's inclusive chunk
-// prefix of site s, so the site is the number of lanes whose prefix the chunk has passed.
-__device__ __forceinline__ void load_chunk(const BatchSmem& B, int chunk, int nchunk, int incl, int gt, Cand& c) {
+// Chunk `chunk` of the work list: 32 candidates of one site.  Lane l holds where entries l and l + 32 of
+// the list begin (`at0`, `at1`), so the entry is the number of those the chunk has reached, less one.
+// What a lane without a candidate leaves in c does not matter: its type is -1.
+__device__ __forceinline__ void load_chunk(const BatchSmem& B, int chunk, int nchunk, int nsite, int at0, int at1,
+                                           Cand& c) {
   const MoveSmem& M = B.M;
   const DevSystem& S = B.Y.S;
-  c.x = c.y = c.z = c.q = 0.0;
   c.type = -1;
-  c.site = 0;
   if (chunk >= nchunk) return;  // the whole warp
-  const int s = __popc(__ballot_sync(0xffffffffu, chunk >= incl));
-  c.site = s;
-  const int j = ((chunk - M.cpre[s]) << 5) + (threadIdx.x & 31), vl = M.vl[s];
-  if (j < vl) {
-    const int i = M.vb[s] + j;
-    load_site(S.vox_xyzq + i, c);
-    c.type = S.vox_type[i];
-  } else if (j - vl < gt) {
-    const int jg = j - vl;
-    int g = 0;
-    while (g + 1 < B.Y.nspecies && jg >= M.gpre[g + 1]) g++;
-    const int i = B.C.seg_off[g] + (jg - M.gpre[g]);
-    if (i < M.ex_lo || i >= M.ex_hi) {
-      load_site(B.C.gsite + i, c);
-      c.type = B.C.gtype[i];
-    }
+  const int e = __popc(__ballot_sync(0xffffffffu, chunk >= at0)) + __popc(__ballot_sync(0xffffffffu, chunk >= at1)) - 1;
+  const int lane = threadIdx.x & 31;
+  const double4* p;
+  const unsigned char* tp;
+  int i;
+  bool live;
+  if (e < nsite) {
+    const int4 d = M.list[e];
+    const int j = ((chunk - d.x) << 5) + lane;
+    i = d.y + j;
+    live = j < d.z;
+    p = S.vox_xyzq;
+    tp = S.vox_type + i;
+    c.site = e;
+  } else {  // guest sites: a guest's type is the low byte of its int
+    c.site = e - nsite;
+    const int j = ((chunk - M.nfw - c.site * M.gchunks) << 5) + lane;
+    live = j < M.gpre[B.Y.nspecies];
+    i = B.C.seg_off[0] + j;
+    if (B.Y.nspecies > 1)
+#pragma unroll 1
+      for (int g = 1; g < B.Y.nspecies; g++)
+        if (j >= M.gpre[g]) i = B.C.seg_off[g] + (j - M.gpre[g]);
+    live = live && (unsigned)(i - M.ex_lo) >= (unsigned)(M.ex_hi - M.ex_lo);
+    p = B.C.gsite;
+    tp = reinterpret_cast<const unsigned char*>(B.C.gtype + i);
   }
+  p += i;
+  if (live) {
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(c.x), "=d"(c.y), "=d"(c.z), "=d"(c.q) : "l"(p));
+    c.type = *tp;
+  }
+}
+
+// x - nint(x) (halves away from zero) by the rounding of an addition.
+__device__ __forceinline__ double nint_rest(double x) {
+  const double f = x - ((x + kMagic) - kMagic);
+  return fabs(f) == 0.5 ? copysign(0.5, -x) : f;
 }
 
 // This warp's share of the real-space pairs (ewald2 + srfrce over guestlistgen's set): chunks warp,
@@ -776,43 +785,56 @@ __device__ __forceinline__ void load_chunk(const BatchSmem& B, int chunk, int nc
 // latency (two chains, 16 warps, share an SM): a pair is a candidate load, an image, a root, three
 // table reads and two interpolations, each waiting for the last.  So U chunks are in flight: their
 // distances first, then the next U chunks' loads, then their table reads, without a branch in
-// between -- a lane whose candidate is missing or beyond the cut-off reads the table at the cut-off
-// and adds zero.  Energy sums of a move, SM cycles (256 chains of 16 frameworks, 1 A voxels, two
-// chains on most SMs; one chain alone on its SM): 17.8k; 12.6k with one branching candidate a trip and
-// two separate tables, 10.5k; 7.4k with U = 2, 10.9k; 7.5k with 3, 11.2k; 8.1k with 4.
+// between -- a lane whose candidate is missing or beyond the cut-off reads row 0 of the table (no vdW)
+// at the cut-off and adds zero.  Energy sums of a move, SM cycles (one chain an SM / 256 chains, two on
+// most SMs): one branching candidate a trip and separate tables 12.6k / 17.8k; U = 2 7.7k / 10.9k,
+// U = 3 7.3k / 10.8k with the whole launch 4% faster / 4% slower (larger code), U = 4 slower for both.
 template <int KIND, int NT, int U>
 __device__ __forceinline__ void real_space(const BatchSmem& B, double& v1, double& v2) {
   const MoveSmem& M = B.M;
   const DevSystem& S = B.Y.S;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, NW = NT / 32;
-  const int nold = M.nold, nsite = nold + M.nnew, gt = M.gpre[B.Y.nspecies];
-  const int nchunk = M.cpre[nsite], nt1 = S.ntypes + 1;
-  const int incl = lane < nsite ? M.cpre[lane + 1] : 0x7fffffff;
-  const bool sub_old = M.mtype != kInsert && M.mtype != kDelete;
-  const double rcut2 = S.rcut2, rdr = S.rdr_e, rdrv = S.rdr_v;
-  const int tstride = S.tab_stride;
+  const int nold = M.nold, nsite = nold + M.nnew, nchunk = M.nfw + nsite * M.gchunks;
+  auto begins = [&M, nsite](int e) {  // the chunk at which entry e begins
+    return e < nsite ? M.list[e].x : (e < 2 * nsite ? M.nfw + (e - nsite) * M.gchunks : 0x7fffffff);
+  };
+  const int at0 = begins(lane), at1 = begins(lane + 32);
+  const int nminus = M.nnew ? nold : 0;  // a displacement's old sites are subtracted
+  const double rcut2 = S.rcut2, rdr = S.rdr_e;
   // imcon 1 takes the first edge for every axis (images, utility_pack.f:1138-1349)
   const int iy = S.cell.imcon == 1 ? 0 : 1, iz = S.cell.imcon == 1 ? 0 : 2;
-  const double hx = S.cell.h[0], hy = S.cell.h[4 * iy], hz = S.cell.h[4 * iz];
-  const double rx = S.cell.inv[0], ry = S.cell.inv[iy], rz = S.cell.inv[iz];
-  constexpr double kMagic = 6755399441055744.0;  // 1.5 x 2^52: adding it rounds to an integer
   Cand c[U];
 #pragma unroll
-  for (int u = 0; u < U; u++) load_chunk(B, warp + u * NW, nchunk, incl, gt, c[u]);
+  for (int u = 0; u < U; u++) {
+    c[u].x = c[u].y = c[u].z = c[u].q = 0.0;
+    c[u].site = 0;
+  }
+#pragma unroll
+  for (int u = 0; u < U; u++) load_chunk(B, warp + u * NW, nchunk, nsite, at0, at1, c[u]);
+#pragma unroll 1
   for (int base = warp; base < nchunk; base += U * NW) {
-    double rs[U], cq[U], sg[U];
-    int off[U];
+    double rs[U], cq[U];
+    int off[U], site[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const int s = c[u].site;
       double dx = M.x[s] - c[u].x, dy = M.y[s] - c[u].y, dz = M.z[s] - c[u].z;
       if (KIND == kPairOrtho) {
         // nint by the rounding of an addition: a tie picks either image, at the same distance
-        dx = fma(-hx, (fma(rx, dx, kMagic) - kMagic), dx);
-        dy = fma(-hy, (fma(ry, dy, kMagic) - kMagic), dy);
-        dz = fma(-hz, (fma(rz, dz, kMagic) - kMagic), dz);
+        const double* hh = S.cell.h;
+        const double* ri = S.cell.inv;
+        dx = fma(-hh[0], fma(ri[0], dx, kMagic) - kMagic, dx);
+        dy = fma(-hh[4 * iy], fma(ri[iy], dy, kMagic) - kMagic, dy);
+        dz = fma(-hh[4 * iz], fma(ri[iz], dz, kMagic) - kMagic, dz);
       } else if (KIND == kPairTriclinic) {
-        min_image_t<3>(S.cell, dx, dy, dz);
+        const double* r = S.cell.rh;
+        const double* hh = S.cell.h;
+        const double fx = nint_rest(r[0] * dx + r[3] * dy + r[6] * dz);
+        const double fy = nint_rest(r[1] * dx + r[4] * dy + r[7] * dz);
+        const double fz = nint_rest(r[2] * dx + r[5] * dy + r[8] * dz);
+        dx = hh[0] * fx + hh[3] * fy + hh[6] * fz;
+        dy = hh[1] * fx + hh[4] * fy + hh[7] * fz;
+        dz = hh[2] * fx + hh[5] * fy + hh[8] * fz;
       } else {
         min_image(S.cell, dx, dy, dz);
       }
@@ -821,29 +843,29 @@ __device__ __forceinline__ void real_space(const BatchSmem& B, double& v1, doubl
       const double qq = M.cq[s] * c[u].q;
       rs[u] = in ? rsq : rcut2;
       cq[u] = in && fabs(qq) > 1e-10 ? qq : 0.0;  // ewald2 skips smaller products
-      const int row = in ? B.prow[M.type[s] * nt1 + c[u].type] : -1;
-      off[u] = row > 0 ? row * tstride : 0;
-      sg[u] = row < 0 ? 0.0 : (sub_old && s < nold ? -1.0 : 1.0);
+      off[u] = in ? B.prow[M.type[s] + c[u].type] : 0;
+      site[u] = s;
     }
 #pragma unroll
-    for (int u = 0; u < U; u++) load_chunk(B, base + (U + u) * NW, nchunk, incl, gt, c[u]);
+    for (int u = 0; u < U; u++) load_chunk(B, base + (U + u) * NW, nchunk, nsite, at0, at1, c[u]);
 #pragma unroll
     for (int u = 0; u < U; u++) {
+      const double sg = site[u] < nminus ? -1.0 : 1.0;
       const double r = sqrt_approx(rs[u]);
       const double x = __dmul_rn(r, rdr);
-      const double t = (x - 0.5) + kMagic;  // floor(x) but for integers, where either interval agrees
-      const int l = __double2loint(t);
-      const double p = x - (t - kMagic), pm = p - 1.0, hp = 0.5 * p;
+      const double f = (x - 0.5) + kMagic;  // floor(x) but for integers, where either interval agrees
+      const int l = __double2loint(f);
+      const double p = x - (f - kMagic), pm = p - 1.0, hp = 0.5 * p;
       if (KIND != kPairGeneral) {
         const double2* tb = S.pair_tab + (off[u] + l);
         const double2 a0 = tb[0], a1 = tb[1], a2 = tb[2];
         const double e1 = fma(a1.x - a0.x, p, a0.x), e2 = fma(a2.x - a1.x, pm, a1.x);
         const double w1 = fma(a1.y - a0.y, p, a0.y), w2 = fma(a2.y - a1.y, pm, a1.y);
         v1 = fma(fma(e2 - e1, hp, e1), cq[u], v1);
-        v2 = fma(fma(w2 - w1, hp, w1), sg[u], v2);
+        v2 = fma(fma(w2 - w1, hp, w1), sg, v2);
       } else {
         v1 = fma(interp3(S.erc, r, rdr), cq[u], v1);
-        if (sg[u] != 0.0) v2 = fma(interp3(S.vvv + off[u], r, rdrv), sg[u], v2);
+        if (off[u]) v2 = fma(interp3(S.vvv + off[u], r, S.rdr_v), sg, v2);
       }
     }
   }
@@ -859,18 +881,20 @@ __device__ __noinline__ void real_space_residue(double* vout) {
   const BatchSmem& B = batch_smem();
   const MoveSmem& M = B.M;
   const DevSystem& S = B.Y.S;
-  const int gt = M.gpre[B.Y.nspecies], T0 = M.vl[0] + gt, T = T0 + M.vl[1] + gt, nt1 = S.ntypes + 1;
+  const int gt = M.gpre[B.Y.nspecies], T0 = M.list[0].z + gt, T = T0 + M.list[1].z + gt;
   const double chgea = B.Y.sp[M.g].q[0] * kR4pie0;
   double v1 = 0.0, v2 = 0.0;
+#pragma unroll 1
   for (int t = threadIdx.x; t < T; t += NT) {
     const int s = t >= T0, j = t - (s ? T0 : 0);
     double4 a;
     int type;
-    if (j < M.vl[s]) {
-      a = S.vox_xyzq[M.vb[s] + j];
-      type = S.vox_type[M.vb[s] + j];
+    const int4 d = M.list[s];
+    if (j < d.z) {
+      a = S.vox_xyzq[d.y + j];
+      type = S.vox_type[d.y + j];
     } else {
-      const int jg = j - M.vl[s];
+      const int jg = j - d.z;
       int g = 0;
       while (g + 1 < B.Y.nspecies && jg >= M.gpre[g + 1]) g++;
       const int i = B.C.seg_off[g] + (jg - M.gpre[g]);
@@ -878,9 +902,24 @@ __device__ __noinline__ void real_space_residue(double* vout) {
       a = B.C.gsite[i];
       type = B.C.gtype[i];
     }
-    const int row = B.prow[M.type[s] * nt1 + type];
+    const int off = B.prow[M.type[s] + type];
     double ec = 0.0, ev = 0.0;
-    pair_energy(S, M.x[s] - a.x, M.y[s] - a.y, M.z[s] - a.z, chgea, a.w, row, ec, ev);
+    double dx = M.x[s] - a.x, dy = M.y[s] - a.y, dz = M.z[s] - a.z;
+    min_image(S.cell, dx, dy, dz);
+    const double rsq = fma(dz, dz, fma(dx, dx, dy * dy));
+    if (rsq < S.rcut2) {
+      const double r = sqrt(rsq), chgprd = chgea * a.w;
+      auto interp = [r](const double* tab, double rdr) {
+        const double x = __dmul_rn(r, rdr);
+        const int l = (int)x;
+        const double p = __dsub_rn(x, (double)l);
+        const double t0 = tab[l], t1 = tab[l + 1], t2 = tab[l + 2];
+        const double u1 = fma(t1 - t0, p, t0), u2 = fma(t2 - t1, p - 1.0, t1);
+        return fma(__dmul_rn(u2 - u1, p), 0.5, u1);
+      };
+      if (fabs(chgprd) > 1e-10) ec = __dmul_rn(interp(S.erc, S.rdr_e), chgprd);
+      if (off) ev = interp(S.vvv + off, S.rdr_v);
+    }
     if (s == 0) {
       v1 -= ec;
       v2 -= ev;
@@ -904,10 +943,12 @@ __device__ __noinline__ void sums_kind(int kmax_smem, int stride) {
   auto term = [&](int k) { return recip_term(k, nsite, k1, k2, stride, A.tab, A.kp, A.ak, A.Sk, A.Sn); };
   int k = tid;
   if (KPT == 2)
+#pragma unroll 1
     for (; k + NT < K; k += 2 * NT) {  // two independent k-vectors in flight, added in order
       const double2 a = term(k), b = term(k + NT);
       v0 = fma(b.x, b.y, fma(a.x, a.y, v0));
     }
+#pragma unroll 1
   for (; k < K; k += NT) {
     const double2 a = term(k);
     v0 = fma(a.x, a.y, v0);
@@ -918,9 +959,9 @@ __device__ __noinline__ void sums_kind(int kmax_smem, int stride) {
     v1 = v[0];
     v2 = v[1];
   } else {
-    real_space<KIND, NT, kChunksPerTrip * CPT>(B, v1, v2);
+    real_space<KIND, NT, kChunksPerTrip + CPT>(B, v1, v2);
   }
-#pragma unroll
+#pragma unroll 1
   for (int o = 16; o > 0; o >>= 1) {
     v0 += __shfl_down_sync(0xffffffffu, v0, o);
     v1 += __shfl_down_sync(0xffffffffu, v1, o);
@@ -940,6 +981,90 @@ __device__ __forceinline__ void sums(const DevSystem& S, int kmax_smem, int stri
   if (S.pair_tab && imcon <= 2) sums_kind<kPairOrtho, NT, KPT, CPT>(kmax_smem, stride);
   else if (S.pair_tab && imcon == 3) sums_kind<kPairTriclinic, NT, KPT, CPT>(kmax_smem, stride);
   else sums_kind<kPairGeneral, NT, KPT, CPT>(kmax_smem, stride);
+}
+
+// Energy assembly of the move (gcmc.f:946, 1112, 1328) from the block's sums {sum akk d|S|^2, ewld2, vdw}.
+__device__ __forceinline__ void assemble(const SysConst& Y, const MoveCtl& T, double v0, double v1, double v2,
+                                         double& ewld1, double& ewld3, double& delrc, double& estep) {
+  const SpeciesConst& P = Y.sp[T.g];
+  ewld1 = Y.S.recip_pref * v0;
+  ewld3 = 0.0;
+  delrc = 0.0;
+  if (T.need_lrc) {
+    delrc = T.lrc - T.elrc;
+    ewld3 = P.ewald3en;
+    const double sg = T.mtype == kInsert ? 1.0 : -1.0;
+    ewld1 = ewld1 + sg * P.engsic;
+    estep = (ewld1 + sg * v1 + sg * ewld3 + sg * v2 + delrc) / Y.engunit;
+  } else {
+    estep = (ewld1 + v1 + v2) / Y.engunit;
+  }
+}
+
+// Acceptance (energy_eval, utility_pack.f:3049-3095, with the displacement shortcut of
+// gcmc.f:1330-1338); `drawn`: the test took the move's acceptance draw, exactly where the reference
+// draws it.
+__device__ __forceinline__ bool decide(double beta, const MoveCtl& T, double e, bool& drawn) {
+  drawn = false;
+  if (T.mtype == kNoop) return false;    // nothing to accept or reject; no draw
+  if (T.mj_stage == 1) return true;      // the first jump is kept for now
+  if (T.mj_stage == 2) e = T.mj_estep + e;  // one test on the summed change (gcmc.f:1730-1739)
+  if (!T.need_lrc && e < 0.0) return true;
+  drawn = true;
+  double test;
+  if (-1 * beta * e > 700.0) {
+    test = exp(700.0);
+  } else {
+    test = exp(-1.0 * beta * e);
+    if (T.need_lrc) test = T.mtype == kDelete && T.free_delete ? 1.0 : T.pref * test;
+  }
+  return T.rande < test;
+}
+
+// Warp 0, once a move is decided: the counters the next set-up reads and the guest sites of an accepted
+// insertion or displacement (an accepted deletion's shift is the whole block's).
+__device__ __forceinline__ void commit_control(const MoveCtl& T, bool accepted, int lane) {
+  BatchSmem& B = batch_smem();
+  ChainDev& C = B.C;
+  MoveSmem& M = B.M;
+  const int mtype = T.mtype, g = T.g, ns = T.ns;
+  const SpeciesConst& P = B.Y.sp[g];
+  if (!accepted) {
+    if (T.mj_stage == 2 && lane < ns)
+      C.gsite[M.mj_lo + lane] =
+          make_double4(M.mj_old[3 * lane], M.mj_old[3 * lane + 1], M.mj_old[3 * lane + 2], P.q[lane]);
+    __syncwarp();
+    return;
+  }
+  if (lane == 0) {
+    if (T.need_lrc) {
+      const int d = mtype == kInsert ? 1 : -1;
+      C.nmol[g] += d;
+      C.totatm += d * ns;
+#pragma unroll 1
+      for (int i = 0; i < ns; i++) C.numtyp[P.type[i]] += d;
+    } else if (mtype == kTranslate) {
+      C.accept_tran[g]++;
+    } else if (mtype == kRotate) {
+      C.accept_rota++;
+    } else if (mtype == kDisplace) {
+      C.accept_disp[g]++;
+    }
+    if (T.mj_stage == 1) M.mj_lo = T.lo;
+  }
+  if (lane < ns) {
+    if (T.mj_stage == 1) {
+      M.mj_old[3 * lane] = M.x[lane];
+      M.mj_old[3 * lane + 1] = M.y[lane];
+      M.mj_old[3 * lane + 2] = M.z[lane];
+    }
+    if (mtype != kDelete) {
+      const int st = mtype == kInsert ? lane : ns + lane;
+      C.gsite[T.lo + lane] = make_double4(M.x[st], M.y[st], M.z[st], P.q[lane]);
+      C.gtype[T.lo + lane] = P.type[lane];
+    }
+  }
+  __syncwarp();
 }
 
 // All threads, in production: storeprob (utility_pack.f:496-561) for the chain's state after the
@@ -1011,7 +1136,8 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 4 : (NT <= 256 ? 2 : 1)) fmc_b
   const SysConst& Y = Ysm;
   const int K = S.K, kmax_smem = L.kmax_smem;
   const int nt1 = S.ntypes + 1;
-  for (int i = tid; i < nt1 * nt1; i += blockDim.x) B.prow[i] = S.pair_row[i];
+  // the offset of each pair's vdW row in the tables, 0 for pairs without one (row 0 is none's)
+  for (int i = tid; i < nt1 * nt1; i += blockDim.x) B.prow[i] = max(S.pair_row[i], 0) * S.tab_stride;
   const BatchArrays A = batch_arrays(kmax_smem);
   double2 *const Sk = A.Sk, *const Sn = A.Sn, *const tab = A.tab;
   for (int k = tid; k < K; k += blockDim.x) {
@@ -1028,28 +1154,70 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 4 : (NT <= 256 ? 2 : 1)) fmc_b
   // out (the reference's do-while(lgchk) loop, gcmc.f:589-736), or at its move budget
   long long nmoves = C.lgchk ? L.moves : 0;
   if (C.budget > 0) nmoves = min(nmoves, C.budget - C.moves_done);
-  if (tid == 0) M.mj_stage = 0;
-  bool pending = false;  // the first half of a multi-jump ended the last trip; the move goes on
+  MoveRecord* trace = L.trace ? L.trace + (size_t)cidx * L.moves : nullptr;
+  if (tid < kMaxGuestTypes) B.st_nmol[tid] = C.nmol[tid];
+  __syncthreads();
+  bool undone = false;  // the last trip's bookkeeping is still to be done
+  bool second = false;  // the last trip was the first half of a multi-jump; the move goes on
+  int skip = 0;         // the last acceptance test took a draw
+  int par = 0;
   for (int mv = 0; mv < nmoves;) {
+    MoveCtl& T = B.ctl[par];
     if (prof && tid == 0) t0 = clock64();
+    // ---- set-up, four warps side by side: 0 draws, selects and builds the trial; 1 finishes the last
+    // move and begins this one (the order of gcmc.f:589-736); 2 builds the phase tables from warp
+    // 0's sites; 3 the tail correction from warp 0's counts.  Named barriers 1 and 2 are warp 0's
+    // signals that the selection and the sites are there.
     if (warp == 0) {
-      if (lane == 0) select_move<kProf>(C, Y, M);
-      __syncwarp();
-      // warp 1 may read select_move's results now (named barrier 1: warps 0 and 1)
-      asm volatile("bar.arrive 1, 64;" ::: "memory");
-      if (!C.status) build_trial<kProf>(C, Y, S, M, tab, stride, lane);
+      select_move(par, skip, second, lane);
+      if (prof && lane == 0) C.prof[7] += clock64() - t0;
+      asm volatile("bar.arrive 1, 96;" ::: "memory");
+      if (prof && lane == 0) t1 = clock64();
+      build_trial(lane);
+      if (prof && lane == 0) C.prof[8] += clock64() - t1;
     } else if (warp == 1) {
-      asm volatile("bar.sync 1, 64;" ::: "memory");
-      if (M.need_lrc && !C.status) lrc_warp(C, Y, M, lane);
+      if (undone) finish_move(trace, lane);
+      if (lane == 0 && !second) {
+        C.gcmccount++;
+        if (C.gcmccount % 400 == 0) check400();
+      }
+      __syncwarp();
+      asm volatile("bar.sync 1, 96;" ::: "memory");
+      if (lane == 0) {
+        T.elrc = C.elrc;
+        T.mj_estep = M.mj_estep;
+        // energy_eval's factor (utility_pack.f:3049-3095) of exp(-beta dE)
+        const double press = C.press[T.g];
+        const bool ins = T.mtype == kInsert;
+        const double vp = Y.statvolm * press, nt = (T.nmols + (ins ? 1 : 0)) * kBoltz * C.temp;
+        T.pref = (ins ? vp : nt) / (ins ? nt : vp);
+        T.free_delete = fabs(press) < 1e-7;
+      }
+    } else if (warp == 2) {
+      asm volatile("bar.sync 2, 64;" ::: "memory");
+      build_phases(B, tab, stride, lane);
+    } else if (warp == 3) {
+      asm volatile("bar.sync 1, 96;" ::: "memory");
+      if (T.need_lrc) lrc_warp(B, M, T.g, T.mtype == kInsert ? 1 : -1, T.lrc, lane);
     }
+    undone = false;
     __syncthreads();
     if (prof && tid == 0) {
       t1 = clock64();
       C.prof[0] += t1 - t0;
       t0 = t1;
     }
-    if (C.status) break;
-    const bool last = !C.lgchk;  // lane 0 of warp 0 writes lgchk only in select_move
+    if (C.status) {
+      if (tid == 0) {  // the move that could not be tried was still counted
+        if (T.mtype == kInsert) C.ins_count++;
+        else if (T.mtype == kDelete) C.del_count++;
+        else if (T.mtype == kJump || T.mj_stage == 1) C.jump_count++;
+      }
+      skip = 0;
+      break;
+    }
+    // read before the sums: the bookkeeping of this move may change them while slow warps commit
+    const bool last = !C.lgchk, store = Y.nplots && C.production;
     sums<NT, KPT, CPT>(S, kmax_smem, stride);
     if (prof && tid == 0) C.prof[6] += clock64() - t0;
     __syncthreads();
@@ -1058,66 +1226,88 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 4 : (NT <= 256 ? 2 : 1)) fmc_b
       C.prof[2] += t1 - t0;
       t0 = t1;
     }
-    if (tid == 0) {
-      double v[3] = {0.0, 0.0, 0.0};
-      for (int w = 0; w < NT / 32; w++)
-        for (int k = 0; k < 3; k++) v[k] += B.red[3 * w + k];
-      assemble(Y, M, v);
-      decide(C, Y, M);
+    // ---- acceptance, by every thread from the warps' sums: no barrier before the commit
+    const int mtype = T.mtype, g = T.g, mj_stage = T.mj_stage;
+    bool accepted, drawn;
+    {
+      double v0 = 0.0, v1 = 0.0, v2 = 0.0;
+#pragma unroll
+      for (int w = 0; w < NT / 32; w++) {
+        v0 += B.red[3 * w];
+        v1 += B.red[3 * w + 1];
+        v2 += B.red[3 * w + 2];
+      }
+      double ewld1, ewld3, delrc, e;
+      assemble(Y, T, v0, v1, v2, ewld1, ewld3, delrc, e);
+      accepted = decide(C.beta, T, e, drawn);
+      if (tid == 32) {
+        MoveDone& D = B.done;
+        D.mtype = mtype;
+        D.g = g;
+        D.randchoice = T.randchoice;
+        D.accepted = accepted;
+        D.mj_stage = mj_stage;
+        D.mv = mv;
+        D.ewld1 = ewld1;
+        D.ewld2 = v1;
+        D.ewld3 = ewld3;
+        D.vdw = v2;
+        D.delrc = delrc;
+        D.estep = e;
+        D.rande = drawn ? T.rande : -1.0;
+      }
     }
-    __syncthreads();
-    if (tid == 0) bookkeep(C, Y, M, L.trace ? L.trace + (size_t)cidx * L.moves + mv : nullptr);
-    __syncthreads();
+    skip = drawn;
+    second = mj_stage == 1;
+    undone = true;
+    par ^= 1;
     if (prof && tid == 0) {
       t1 = clock64();
       C.prof[3] += t1 - t0;
       t0 = t1;
     }
-    if (M.mj_action == 1)  // park S(k) before the first jump of a multi-jump is committed
-      for (int k = tid; k < K; k += blockDim.x) C.sk[k] = Sk[k];
-    if (M.mj_action == 2) {  // rejected multi-jump: S(k) and the first molecule as they were
-      for (int k = tid; k < K; k += blockDim.x) Sk[k] = C.sk[k];
-      if (tid < M.ns)
-        C.gsite[M.mj_lo + tid] =
-            make_double4(M.mj_old[3 * tid], M.mj_old[3 * tid + 1], M.mj_old[3 * tid + 2], Y.sp[M.g].q[tid]);
-    }
-    if (M.accepted) {
-      for (int k = tid; k < K; k += blockDim.x) Sk[k] = Sn[k];
-      const int ns = M.ns, mtype = M.mtype;
-      if (mtype == kDelete) {
-        const int lo = M.commit_lo, end = M.seg_end;
-        for (int base = lo; base < end - ns; base += blockDim.x) {
-          int i = base + tid;
-          bool act = i < end - ns;
-          double4 a = make_double4(0, 0, 0, 0);
-          int t = 0;
-          if (act) {
-            a = C.gsite[i + ns];
-            t = C.gtype[i + ns];
-          }
-          __syncthreads();
-          if (act) {
-            C.gsite[i] = a;
-            C.gtype[i] = t;
-          }
-          __syncthreads();
+    // ---- commit: every thread its own k-vectors, warp 0 the guest sites and the counts it reads
+    if (second)  // park S(k) before the first jump of a multi-jump is committed
+#pragma unroll 1
+      for (int k = tid; k < K; k += NT) C.sk[k] = Sk[k];
+    if (mj_stage == 2 && !accepted)  // rejected multi-jump: S(k) as it was
+#pragma unroll 1
+      for (int k = tid; k < K; k += NT) Sk[k] = C.sk[k];
+    if (accepted)
+#pragma unroll 1
+      for (int k = tid; k < K; k += NT) Sk[k] = Sn[k];
+    if (accepted && mtype == kDelete) {
+      const int ns = T.ns, lo = T.lo, end = T.seg_end;
+      for (int base = lo; base < end - ns; base += NT) {
+        int i = base + tid;
+        bool act = i < end - ns;
+        double4 a = make_double4(0, 0, 0, 0);
+        int t = 0;
+        if (act) {
+          a = C.gsite[i + ns];
+          t = C.gtype[i + ns];
         }
-      } else if (tid < ns) {
-        int st = (mtype == kInsert) ? tid : ns + tid;
-        C.gsite[M.commit_lo + tid] = make_double4(M.x[st], M.y[st], M.z[st], Y.sp[M.g].q[tid]);
-        C.gtype[M.commit_lo + tid] = M.type[st];
+        __syncthreads();
+        if (act) {
+          C.gsite[i] = a;
+          C.gtype[i] = t;
+        }
+        __syncthreads();
       }
     }
-    // read before the barrier: thread 0 may change these in the next select_move
-    pending = M.mj_stage == 1;
-    const bool store = Y.nplots && C.production && !pending;
-    __syncthreads();
+    if (warp == 0) commit_control(T, accepted, lane);
+    if (store && !second) {  // every production move (gcmc.f:1929-1931)
+      __syncthreads();
+      prob_store(Y, C);
+    }
     if (prof && tid == 0) C.prof[4] += clock64() - t0;
-    if (store) prob_store(Y, C);  // every production move (gcmc.f:1929-1931)
-    if (pending) continue;
+    if (second) continue;
     if (last) break;
     mv++;
   }
+  if (warp == 1 && undone) finish_move(trace, lane);
+  if (tid == 0 && skip) duni_next(C.rng);
+  __syncthreads();
   for (int k = tid; k < K; k += blockDim.x) C.sk[k] = Sk[k];
   if (tid == 0 && L.retire_finished && ((C.budget > 0 && C.moves_done >= C.budget) || !C.lgchk || C.status))
     C.active = 0;

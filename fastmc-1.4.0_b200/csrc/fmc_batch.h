@@ -25,8 +25,8 @@ constexpr int kBatchMaxTab = kBatchMaxTypes * (kBatchMaxTypes + 1) / 2;
 struct BatchTile {
   int threads, kvec_per_trip, cand_per_trip;
 };
-// Chunks of 32 candidates a warp has in flight in the real-space loop, per candidate of the tile.
-constexpr int kChunksPerTrip = 2;
+// Chunks of 32 candidates a warp has in flight in the real-space loop, beyond the tile's candidates.
+constexpr int kChunksPerTrip = 1;
 constexpr int kNumBatchTiles = 12;
 constexpr BatchTile kBatchTiles[kNumBatchTiles] = {
     {256, 1, 1}, {256, 2, 1}, {256, 1, 2}, {256, 2, 2}, {128, 1, 1}, {128, 2, 1},
@@ -116,6 +116,8 @@ struct BatchLaunch {
 };
 
 cudaError_t launch_batch(const BatchLaunch& L, int smem_bytes, int tab_stride, cudaStream_t st);
+// Shared memory a CTA may take on sm_100.
+constexpr int kBatchMaxSmem = 227 * 1024;
 int batch_smem_bytes(int kmax_K, int tab_sites, int tab_stride);
 cudaError_t configure_batch_kernel(int smem_bytes);
 

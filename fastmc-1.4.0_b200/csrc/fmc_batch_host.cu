@@ -281,7 +281,7 @@ int Batch::open(const std::vector<std::string>& dirs, const std::vector<int>& se
   }
   kmax_all = (kmax_all + 3) & ~3;
   smem = batch_smem_bytes(kmax_all, tab_sites, tab_stride);
-  if (smem > 227 * 1024) {
+  if (smem > kBatchMaxSmem) {
     err = "k-vector tables of this batch exceed the shared-memory budget of one CTA";
     return -9;
   }

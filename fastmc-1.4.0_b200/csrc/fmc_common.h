@@ -498,20 +498,24 @@ struct WindowStats {
   double seltot[kMaxGuestTypes][kMaxGuestTypes], selwin[kMaxGuestTypes][kMaxGuestTypes];
 };
 
+// The rolling <exp(-dE/kT)> of an accepted insertion of species i (cs[5], window mean avg[7]).
+FMC_HD void window_insertion(WindowStats& W, int i, double delE, double temp, int accept_ins, double* cs) {
+  double* aw = W.avg[i];
+  double h = exp(-1.0 * delE / kKboltz / temp);
+  W.ins_rollcount++;
+  double delta = h - cs[5];
+  h = cs[5] + delta / accept_ins;
+  cs[5] = h;
+  aw[7] = ((W.ins_rollcount - 1) * aw[7] + h) / (double)W.ins_rollcount;
+}
+
 // One counted production sample of species i, after its cumulative averages cs[0..4] (<N>,
 // <E>, <EN>, <N^2>, <E^2>) were updated; cs[5] is the rolling <exp(-dE/kT)> of accepted
 // insertions.  rollcount must already count this sample.
 FMC_HD void window_sample(WindowStats& W, int i, double dm, double e, bool ins_accepted, double delE, double temp,
                           int accept_ins, double* cs) {
   double* aw = W.avg[i];
-  if (ins_accepted) {
-    double h = exp(-1.0 * delE / kKboltz / temp);
-    W.ins_rollcount++;
-    double delta = h - cs[5];
-    h = cs[5] + delta / accept_ins;
-    cs[5] = h;
-    aw[7] = ((W.ins_rollcount - 1) * aw[7] + h) / (double)W.ins_rollcount;
-  }
+  if (ins_accepted) window_insertion(W, i, delE, temp, accept_ins, cs);
   const double rc = (double)W.rollcount;
   aw[0] = ((W.rollcount - 1) * aw[0] + dm) / rc;
   aw[1] = ((W.rollcount - 1) * aw[1] + e) / rc;

@@ -75,6 +75,7 @@ __device__ __forceinline__ void axis_phases(double s, int kmax, double2* tab, do
   tab[0] = make_double2(q, 0.0);
   double2 p = make_double2(q * cs, q * sn);
   if (kmax >= 1) tab[1] = p;
+#pragma unroll 1
   for (int j = 2; j <= kmax; j++) {
     p = make_double2(p.x * cs - p.y * sn, p.y * cs + p.x * sn);
     tab[j] = p;

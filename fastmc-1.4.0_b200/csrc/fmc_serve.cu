@@ -103,7 +103,7 @@ class Server {
   static constexpr int kServeMaxSites = 4;
   int device = 0;
   cudaStream_t st = nullptr;
-  int nslots = 0, kcap = 0, tab_sites = 2 * kServeMaxSites, tab_stride = 0, smem = 0;
+  int nslots = 0, kcap = 0, tab_sites = 2 * kServeMaxSites, tab_stride = 0;
   size_t budget = 0;
   std::atomic<size_t> used{0};      // device bytes of admitted slots
   size_t prebuilt_bytes = 0;        // device bytes of slots built ahead (guarded by mu)
@@ -211,12 +211,11 @@ class Server {
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
     budget = mem_budget ? mem_budget : (size_t)(0.8 * (double)free_b);
-    smem = batch_smem_bytes(kcap, tab_sites, tab_stride);
-    if (smem > 227 * 1024) {
+    if (batch_smem_bytes(kcap, tab_sites, tab_stride) > kBatchMaxSmem) {
       err = "k-vector capacity exceeds the shared-memory budget of one CTA";
       return -9;
     }
-    if (configure_batch_kernel(smem) != cudaSuccess || configure_kernels() != cudaSuccess ||
+    if (configure_batch_kernel(kBatchMaxSmem) != cudaSuccess || configure_kernels() != cudaSuccess ||
         configure_recip_kernels() != cudaSuccess) {
       err = "cannot configure the kernels";
       return -100;
@@ -937,7 +936,18 @@ class Server {
     L.systems = d_sys;
     L.nchains = nslots;
     L.moves = moves;
-    L.kmax_smem = kcap;
+    // shared memory for the requests in this launch, not for the largest the server admits: what a CTA
+    // leaves is L1 for the tables' gathers, and below half an SM's a second CTA fits beside it
+    int kmax = 4, sites = 1, axes = 3;
+    for (int i = 0; i < nslots; i++)
+      if (slots[i].request >= 0) {
+        const SysConst& Y = h_sys[i];
+        kmax = std::max(kmax, (Y.S.K + 3) & ~3);
+        axes = std::max(axes, Y.S.kmax[0] + Y.S.kmax[1] + Y.S.kmax[2] + 3);
+        for (int g = 0; g < Y.nspecies; g++) sites = std::max(sites, 2 * Y.sp[g].nsite);
+      }
+    L.kmax_smem = kmax;
+    const int smem = batch_smem_bytes(kmax, sites, axes);
     L.retire_finished = 1;
     if (e == cudaSuccess) e = cudaEventRecord(ev_start[b], st);
     if (e == cudaSuccess) e = launch_batch(L, smem, tab_stride, st);
