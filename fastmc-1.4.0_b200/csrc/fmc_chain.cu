@@ -120,6 +120,10 @@ int upload_system(const HostSystem& h, DeviceSystem& d, std::string& err) {
     std::vector<int> kp(h.K);
     for (int k = 0; k < h.K; k++) kp[k] = kpack(h.kl[k], h.km[k], h.kn[k]);
     if ((e = upload(d.allocations, &v.kpack, kp)) != cudaSuccess) goto fail;
+    std::vector<KOctet> oct;
+    recip_octets(kp.data(), h.K, oct);
+    v.noct = (int)oct.size();
+    if ((e = upload(d.allocations, &v.koct, oct)) != cudaSuccess) goto fail;
   }
   if ((e = upload(d.allocations, &v.akk, h.akk)) != cudaSuccess) goto fail;
   v.recip_pref = h.recip_pref;
@@ -179,8 +183,9 @@ Chain::~Chain() {
     if (d_fl) cudaFree(d_fl);
     cudaStreamSynchronize(st);
     for (void* p : {(void*)sk, (void*)sk_new, (void*)sk_save, (void*)gsite, (void*)gtype, (void*)W.recip_part, (void*)W.site_e,
-                    (void*)W.counter, (void*)recip_scratch, (void*)recip_parts, (void*)all_atoms})
+                    (void*)W.counter, (void*)recip_scratch, (void*)sp_work})
       if (p) cudaFree(p);
+    if (recip_parts) cudaFreeHost(recip_parts);
     if (W.result) cudaFreeHost(W.result);
     cudaStreamDestroy(st);
   }
@@ -273,11 +278,10 @@ int Chain::open_prepared(HostSystem&& prepared, const int seed[4], int dev, std:
   FMC_CUDA(cudaMalloc(&d_fl, sizeof(PassServerFlags)));
   std::memset(mb, 0, sizeof(PassMailbox));
   srv_words[0] = srv_words[1] = 0;
-  all_cap = sys.nf + gcap;
-  FMC_CUDA(cudaMalloc(&all_atoms, sizeof(double4) * std::max(all_cap, 1)));
-  recip_scratch_n = recip_scratch_doubles(dsys.view, all_cap);
+  recip_scratch_n = recip_scratch_doubles(dsys.view, sys.nf + gcap);
   FMC_CUDA(cudaMalloc(&recip_scratch, sizeof(double) * recip_scratch_n));
-  FMC_CUDA(cudaMalloc(&recip_parts, sizeof(double) * (recip_nparts(dsys.view) + 1)));
+  // energy partials in pinned host memory, written by the kernel: no copy back to wait for
+  FMC_CUDA(cudaMallocHost(&recip_parts, sizeof(double) * (recip_nparts(dsys.view) + 1)));
   // upload preloaded guests
   for (int g = 0; g < ng; g++) {
     rc = set_guests(g, sp[g].nmol, sp[g].xyz.data());
@@ -407,20 +411,11 @@ int Chain::restart(const Revive& r, std::string& err) {
 int Chain::full_recip(double* e_out) {
   if (int rc0 = stop_server()) return rc0;  // nothing else runs beside the resident kernel
   if (int rc = flush_commit()) return rc;
-  int n = 0;
-  cudaError_t e = cudaSuccess;
-  for (auto& s : sp) {
-    int len = s.nmol * s.nsite;
-    if (len) e = cudaMemcpyAsync(all_atoms + n, gsite + s.seg_off, sizeof(double4) * len, cudaMemcpyDeviceToDevice, st);
-    n += len;
-  }
-  if (e == cudaSuccess && sys.nf)
-    e = cudaMemcpyAsync(all_atoms + n, dsys.view.fw, sizeof(double4) * sys.nf, cudaMemcpyDeviceToDevice, st);
-  n += sys.nf;
-  if (e == cudaSuccess) e = launch_recip_full(dsys.view, all_atoms, n, sk, recip_scratch, recip_parts, st);
-  std::vector<double> parts(recip_nparts(dsys.view));
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(parts.data(), recip_parts, sizeof(double) * parts.size(), cudaMemcpyDeviceToHost, st);
+  AtomSegs atoms;
+  const int ng = (int)sp.size();
+  for (int g = 0; g < ng; g++) atoms.add(g, gsite + sp[g].seg_off, sp[g].nmol * sp[g].nsite);
+  atoms.add(ng, dsys.view.fw, sys.nf);
+  cudaError_t e = launch_recip_full(dsys.view, atoms, sk, recip_scratch, recip_parts, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return sync_error(e);
   double q2 = 0.0;
@@ -429,7 +424,7 @@ int Chain::full_recip(double* e_out) {
       for (int i = 0; i < sp[g].nsite; i++) q2 = q2 + sys.deck.guests[g].charge[i] * sys.deck.guests[g].charge[i];
   for (int i = 0; i < sys.nf; i++) q2 = q2 + sys.fq[i] * sys.fq[i];
   double engsic = -kR4pie0 * sys.alpha * q2 / kSqrPi;
-  if (e_out) *e_out = recip_energy_from_parts(dsys.view, parts.data()) + engsic;
+  if (e_out) *e_out = recip_energy_from_parts(dsys.view, recip_parts) + engsic;
   return 0;
 }
 
@@ -440,15 +435,14 @@ int Chain::single_point() {
   if (int rc0 = stop_server()) return rc0;  // nothing else runs beside the resident kernel
   if (int rc = flush_commit()) return rc;
   // framework only
-  cudaError_t e = launch_recip_full(dsys.view, dsys.view.fw, sys.nf, sk, recip_scratch, recip_parts, st);
-  std::vector<double> parts(recip_nparts(dsys.view));
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(parts.data(), recip_parts, sizeof(double) * parts.size(), cudaMemcpyDeviceToHost, st);
+  AtomSegs fw;
+  fw.add(0, dsys.view.fw, sys.nf);
+  cudaError_t e = launch_recip_full(dsys.view, fw, sk, recip_scratch, recip_parts, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return sync_error(e);
   double q2f = 0.0;
   for (int i = 0; i < sys.nf; i++) q2f = q2f + sys.fq[i] * sys.fq[i];
-  ewald1sum = recip_energy_from_parts(dsys.view, parts.data()) + (-kR4pie0 * sys.alpha * q2f / kSqrPi);
+  ewald1sum = recip_energy_from_parts(dsys.view, recip_parts) + (-kR4pie0 * sys.alpha * q2f / kSqrPi);
   double eall = 0.0;
   int rc = full_recip(&eall);
   if (rc) return rc;
@@ -480,10 +474,17 @@ int Chain::single_point() {
           hi.push_back(sp[g].seg_off + (m + 1) * sp[g].nsite);
         }
     const int n = (int)idx.size();
-    int* dbuf = nullptr;
-    double* dout = nullptr;
-    e = cudaMalloc(&dbuf, sizeof(int) * 3 * n);
-    if (e == cudaSuccess) e = cudaMalloc(&dout, sizeof(double) * 4 * n);
+    // workspace of the chain's own, grown when the guests need more of it
+    const size_t need = sizeof(double) * 4 * n + sizeof(int) * 3 * n;
+    if (need > sp_cap) {
+      if (sp_work) cudaFree(sp_work);
+      sp_work = nullptr;
+      sp_cap = 0;
+      e = cudaMalloc(&sp_work, need + need / 2);
+      if (e == cudaSuccess) sp_cap = need + need / 2;
+    }
+    double* dout = sp_work;
+    int* dbuf = reinterpret_cast<int*>(sp_work + 4 * (size_t)n);
     std::vector<int> packed;
     packed.insert(packed.end(), idx.begin(), idx.end());
     packed.insert(packed.end(), lo.begin(), lo.end());
@@ -493,8 +494,6 @@ int Chain::single_point() {
     std::vector<double> out(4 * n);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out.data(), dout, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(dbuf);
-    cudaFree(dout);
     if (e != cudaSuccess) return sync_error(e);
     double cf = 0, vf = 0, cg = 0, vg = 0;
     for (int i = 0; i < n; i++) {

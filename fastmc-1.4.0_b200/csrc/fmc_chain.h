@@ -54,10 +54,10 @@ class Chain {
   int gcap = 0;
   PassScratch W{};
   double* recip_scratch = nullptr;
-  double* recip_parts = nullptr;
+  double* recip_parts = nullptr;  // pinned
   size_t recip_scratch_n = 0;
-  double4* all_atoms = nullptr;
-  int all_cap = 0;
+  double* sp_work = nullptr;  // single-point workspace, grown when a call needs more
+  size_t sp_cap = 0;
   // host mirror
   std::vector<Species> sp;
   int totatm = 0, framatm = 0;

@@ -37,8 +37,17 @@ struct DevSystem {
   int K;
   int kmax[3];
   const int* kpack;
+  const struct KOctet* koct;  // the k-vectors by (l, |m|) and pairs of |n|
+  int noct;
   const double* akk;
   double recip_pref;
+};
+
+// The k-vectors (l, +-m, +-n) of two |n|: table indices in the order (+m,+n), (+m,-n), (-m,+n), (-m,-n)
+// of n[0], then of n[1]; -1 where the half space or the cut-off leaves one out.
+struct KOctet {
+  int k[8];
+  short l, m, n[2];
 };
 
 constexpr int kMaxPassSites = 2 * kMaxGuestSites;

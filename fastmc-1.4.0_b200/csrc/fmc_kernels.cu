@@ -11,9 +11,11 @@
 // fmc_commit_kernel : S(k) <- S_new and the guest-site array update of an accepted move.
 // fmc_recip_*       : full S(k) of a set of atoms (ewald1, ewald.f:368-630).
 // fmc_sp_kernel     : per-guest-site real-space energies for the single-point energy.
+#include <algorithm>
 #include <cmath>
 #include <cstddef>
 #include <cstring>
+#include <vector>
 
 #include "fmc_device.cuh"
 #include "fmc_kernels.h"
@@ -412,62 +414,155 @@ cudaError_t launch_commit(int K, double2* sk, const double2* sk_new, const Commi
 }
 
 // ------------------------------------------------------------------------------ full S(k)
-// partial[c*K + k] = sum over the atoms of chunk c (in order) of q e^{i k.r}
-constexpr int kRecipThreads = 128;
+// partial[c*K + k] = sum over the atoms of chunk c (in order) of q e^{i k.r}, the chunks then added in
+// order: one fixed order of additions, on which the last bits of S(k) depend.
+//
+// Two forms with the same bits (products are written as the compiler contracted the plain expressions):
+//
+// fmc_recip_octet_kernel: a thread takes the k-vectors (l, +-m, +-n) and (l, +-m, +-n') of two |n|
+// (S.koct): one read each of the three axes' phases serves all eight, and e^{i(lx +- my)} is formed
+// once for four of them.  128-bit shared reads cost four cycles an SM whatever they hit, so one
+// k-vector a thread is bound by them (12 cycles of reads a k-vector and warp against 5 of FP64); here
+// two cycles of reads against 3.5 of FP64.
+//
+// fmc_recip_single_kernel: one k-vector a thread, for the sizes whose octets would leave SMs idle.
+constexpr int kOctetThreads = 128, kSingleThreads = 256;
 
-__global__ void __launch_bounds__(kRecipThreads) fmc_recip_partial_kernel(DevSystem S, const double4* __restrict__ atoms,
-                                                                          int natoms, int chunk, double2* partial) {
-  extern __shared__ double2 sm_tab[];
-  __shared__ double sq[256];
-  const int k1 = S.kmax[0], k2 = S.kmax[1], k3 = S.kmax[2];
-  const int stride = (k1 + 1) + (k2 + 1) + (k3 + 1);
-  const int c = blockIdx.y, a0 = c * chunk;
-  const int na = min(chunk, natoms - a0);
+// Phase tables and charges of a chunk's atoms.
+__device__ __forceinline__ void recip_phases(const DevSystem& S, const AtomSegs& atoms, int a0, int na, int stride,
+                                             double2* tab, double* sq) {
+  const int k1 = S.kmax[0], k2 = S.kmax[1];
   for (int w = threadIdx.x; w < na * 3; w += blockDim.x) {
-    int s = w / 3, ax = w % 3;
-    double4 a = atoms[a0 + s];
+    int s = w / 3, ax = w % 3, i = a0 + s;
+    const double4* p = atoms.p[0];
+#pragma unroll
+    for (int g = 1; g <= kMaxGuestTypes; g++)
+      if (i >= atoms.begin[g]) p = atoms.p[g] - atoms.begin[g];
+    double4 a = p[i];
     double f[3];
     frac_coords(S.cell, a.x, a.y, a.z, f);
-    double2* t = sm_tab + s * stride + (ax == 0 ? 0 : (ax == 1 ? k1 + 1 : k1 + k2 + 2));
+    double2* t = tab + s * stride + (ax == 0 ? 0 : (ax == 1 ? k1 + 1 : k1 + k2 + 2));
     axis_phases(f[ax], S.kmax[ax], t);
     if (ax == 0) sq[s] = a.w;
   }
   __syncthreads();
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
+}
+
+// acc += q e^{i(lx + my)} e3, e3 conjugated for n < 0.
+template <bool kMinus>
+__device__ __forceinline__ void recip_add(double px, double py, double2 e3, double q, double2& acc) {
+  const double cx = kMinus ? fma(px, e3.x, py * e3.y) : fma(px, e3.x, -(py * e3.y));
+  const double cy = kMinus ? fma(py, e3.x, -(e3.y * px)) : fma(e3.y, px, py * e3.x);
+  acc.x = fma(q, cx, acc.x);
+  acc.y = fma(q, cy, acc.y);
+}
+
+__global__ void __launch_bounds__(kOctetThreads) fmc_recip_octet_kernel(DevSystem S, AtomSegs atoms, int natoms,
+                                                                        int chunk, double2* partial) {
+  extern __shared__ double2 sm_tab[];
+  __shared__ double sq[256];
+  const int k1 = S.kmax[0], k2 = S.kmax[1], stride = k1 + k2 + S.kmax[2] + 3;
+  const int c = blockIdx.y, a0 = c * chunk, na = min(chunk, natoms - a0);
+  recip_phases(S, atoms, a0, na, stride, sm_tab, sq);
+  const int run = blockIdx.x * blockDim.x + threadIdx.x;
+  if (run >= S.noct) return;
+  const KOctet& oct = S.koct[run];
+  const double2 *t1 = sm_tab + oct.l, *t2 = sm_tab + k1 + 1 + oct.m, *t3 = sm_tab + k1 + k2 + 2 + oct.n[0],
+                *t4 = sm_tab + k1 + k2 + 2 + oct.n[1];
+  double2 acc[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) acc[i] = make_double2(0.0, 0.0);
+  for (int s = 0; s < na; s++) {
+    const int o = s * stride;
+    const double2 e1 = t1[o], e2 = t2[o], e3 = t3[o], e4 = t4[o];
+    const double q = sq[s];
+    const double px = fma(e1.x, e2.x, -(e1.y * e2.y)), py = fma(e1.y, e2.x, e2.y * e1.x);
+    const double mx = fma(e1.x, e2.x, e1.y * e2.y), my = fma(e1.y, e2.x, -(e2.y * e1.x));
+    recip_add<false>(px, py, e3, q, acc[0]);
+    recip_add<true>(px, py, e3, q, acc[1]);
+    recip_add<false>(mx, my, e3, q, acc[2]);
+    recip_add<true>(mx, my, e3, q, acc[3]);
+    recip_add<false>(px, py, e4, q, acc[4]);
+    recip_add<true>(px, py, e4, q, acc[5]);
+    recip_add<false>(mx, my, e4, q, acc[6]);
+    recip_add<true>(mx, my, e4, q, acc[7]);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int k = oct.k[i];
+    if (k >= 0) partial[(size_t)c * S.K + k] = acc[i];
+  }
+}
+
+__global__ void __launch_bounds__(kSingleThreads) fmc_recip_single_kernel(DevSystem S, AtomSegs atoms, int natoms,
+                                                                          int chunk, double2* partial) {
+  extern __shared__ double2 sm_tab[];
+  __shared__ double sq[256];
+  const int k1 = S.kmax[0], k2 = S.kmax[1], stride = k1 + k2 + S.kmax[2] + 3;
+  const int c = blockIdx.y, a0 = c * chunk, na = min(chunk, natoms - a0);
+  recip_phases(S, atoms, a0, na, stride, sm_tab, sq);
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= S.K) return;
   int l, m, n;
   kunpack(S.kpack[k], l, m, n);
-  int am = m < 0 ? -m : m, an = n < 0 ? -n : n;
+  const double2 *t1 = sm_tab + l, *t2 = sm_tab + k1 + 1 + (m < 0 ? -m : m),
+                *t3 = sm_tab + k1 + k2 + 2 + (n < 0 ? -n : n);
+  const int mneg = m & 0x80000000;
+  const bool nneg = n < 0;
   double2 acc = make_double2(0.0, 0.0);
+#pragma unroll 4
   for (int s = 0; s < na; s++) {
-    const double2* t = sm_tab + s * stride;
-    double2 e1 = t[l], e2 = t[k1 + 1 + am], e3 = t[k1 + k2 + 2 + an];
-    double2 cc = m >= 0 ? cmul(e1, e2) : cmulc(e1, e2);
-    cc = n >= 0 ? cmul(cc, e3) : cmulc(cc, e3);
-    acc.x += sq[s] * cc.x;
-    acc.y += sq[s] * cc.y;
+    const int o = s * stride;
+    const double2 e1 = t1[o], e2 = t2[o], e3 = t3[o];
+    const double y2 = __hiloint2double(__double2hiint(e2.y) ^ mneg, __double2loint(e2.y));
+    const double px = fma(e1.x, e2.x, -(e1.y * y2)), py = fma(e1.y, e2.x, y2 * e1.x);
+    double2 a = acc, b = acc;
+    recip_add<false>(px, py, e3, sq[s], a);
+    recip_add<true>(px, py, e3, sq[s], b);
+    acc.x = nneg ? b.x : a.x;
+    acc.y = nneg ? b.y : a.y;
   }
   partial[(size_t)c * S.K + k] = acc;
 }
 
-// S[k] = sum_c partial[c][k]; energy sum akk |S|^2 per block into part[]
-__global__ void fmc_recip_reduce_kernel(DevSystem S, const double2* __restrict__ partial, int nchunk, double2* sk,
-                                        double* part) {
-  __shared__ double red[32];
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  double v[1] = {0.0};
+// S[k] = sum_c partial[c][k] in order; energy sum akk |S|^2 per block into part[].  Bound by the latency
+// of its reads: blocks of 32 k-vectors spread a few thousand of them over the SMs, and sixteen chunks
+// are read before they are added.
+constexpr int kRecipReduce = 32;
+
+__global__ void __launch_bounds__(kRecipReduce) fmc_recip_reduce_kernel(DevSystem S, const double2* __restrict__ partial,
+                                                                        int nchunk, double2* sk, double* part) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  double v = 0.0;
   if (k < S.K) {
     double2 s = make_double2(0.0, 0.0);
-    for (int c = 0; c < nchunk; c++) {
-      double2 p = partial[(size_t)c * S.K + k];
-      s.x += p.x;
-      s.y += p.y;
+    const double2* p = partial + k;
+    int c = 0;
+    for (; c + 16 <= nchunk; c += 16) {
+      double2 a[16];
+#pragma unroll
+      for (int u = 0; u < 16; u++) a[u] = __ldcg(p + (size_t)(c + u) * S.K);
+#pragma unroll
+      for (int u = 0; u < 16; u++) {
+        s.x += a[u].x;
+        s.y += a[u].y;
+      }
     }
+    double2 a[15];
+#pragma unroll
+    for (int u = 0; u < 15; u++)
+      if (c + u < nchunk) a[u] = __ldcg(p + (size_t)(c + u) * S.K);
+#pragma unroll
+    for (int u = 0; u < 15; u++)
+      if (c + u < nchunk) {
+        s.x += a[u].x;
+        s.y += a[u].y;
+      }
     sk[k] = s;
-    v[0] = S.akk[k] * (s.x * s.x + s.y * s.y);
+    v = S.akk[k] * (s.x * s.x + s.y * s.y);
   }
-  block_sum<1>(v, red);
-  if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (threadIdx.x == 0) part[blockIdx.x] = v;
 }
 
 int recip_chunk(const DevSystem& S) {
@@ -483,10 +578,11 @@ size_t recip_scratch_doubles(const DevSystem& S, int natoms) {
   return (size_t)nchunk * S.K * 2 + 8;
 }
 
-int recip_nparts(const DevSystem& S) { return (S.K + 255) / 256; }
+int recip_nparts(const DevSystem& S) { return (S.K + kRecipReduce - 1) / kRecipReduce; }
 
-cudaError_t launch_recip_full(const DevSystem& S, const double4* atoms, int natoms, double2* sk, double* scratch,
-                              double* parts, cudaStream_t st) {
+cudaError_t launch_recip_full(const DevSystem& S, const AtomSegs& atoms, double2* sk, double* scratch, double* parts,
+                              cudaStream_t st) {
+  const int natoms = atoms.total();
   int chunk = recip_chunk(S);
   int nchunk = (natoms + chunk - 1) / chunk;
   if (nchunk == 0) {
@@ -495,15 +591,74 @@ cudaError_t launch_recip_full(const DevSystem& S, const double4* atoms, int nato
   }
   int stride = (S.kmax[0] + 1) + (S.kmax[1] + 1) + (S.kmax[2] + 1);
   double2* partial = reinterpret_cast<double2*>(scratch);
-  dim3 g((S.K + kRecipThreads - 1) / kRecipThreads, nchunk);
-  fmc_recip_partial_kernel<<<g, kRecipThreads, chunk * stride * sizeof(double2), st>>>(S, atoms, natoms, chunk,
-                                                                                      partial);
-  fmc_recip_reduce_kernel<<<recip_nparts(S), 256, 0, st>>>(S, partial, nchunk, sk, parts);
+  const size_t smem = chunk * stride * sizeof(double2);
+  // octets once their blocks give every SM one: below that the launch lasts as long as one thread's
+  // atoms, eight times shorter with one k-vector a thread
+  const int bx = (S.noct + kOctetThreads - 1) / kOctetThreads;
+  if (bx * nchunk >= 148)
+    fmc_recip_octet_kernel<<<dim3(bx, nchunk), kOctetThreads, smem, st>>>(S, atoms, natoms, chunk, partial);
+  else
+    fmc_recip_single_kernel<<<dim3((S.K + kSingleThreads - 1) / kSingleThreads, nchunk), kSingleThreads, smem, st>>>(
+        S, atoms, natoms, chunk, partial);
+  fmc_recip_reduce_kernel<<<recip_nparts(S), kRecipReduce, 0, st>>>(S, partial, nchunk, sk, parts);
   return cudaGetLastError();
 }
 
 cudaError_t configure_recip_kernels() {
-  return cudaFuncSetAttribute(fmc_recip_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+  cudaError_t e = cudaFuncSetAttribute(fmc_recip_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(fmc_recip_octet_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+  return e;
+}
+
+void recip_octets(const int* kpacked, int K, std::vector<KOctet>& out) {
+  // quads (l, |m|, |n|) in table order, paired within an (l, |m|)
+  struct Quad {
+    int l, m, n, k[4];
+  };
+  std::vector<Quad> quads;
+  std::vector<int> at(129 * 129, -1);  // (|m|, |n|) of the present l
+  int l0 = -1;
+  for (int k = 0; k < K; k++) {
+    int l, m, n;
+    kunpack(kpacked[k], l, m, n);
+    if (l != l0) {
+      std::fill(at.begin(), at.end(), -1);
+      l0 = l;
+    }
+    const int am = m < 0 ? -m : m, an = n < 0 ? -n : n;
+    int& q = at[am * 129 + an];
+    if (q < 0) {
+      q = (int)quads.size();
+      quads.push_back({l, am, an, {-1, -1, -1, -1}});
+    }
+    quads[q].k[(m < 0 ? 2 : 0) + (n < 0 ? 1 : 0)] = k;
+  }
+  std::sort(quads.begin(), quads.end(), [](const Quad& a, const Quad& b) {
+    return a.l != b.l ? a.l < b.l : (a.m != b.m ? a.m < b.m : a.n < b.n);
+  });
+  out.clear();
+  for (size_t i = 0; i < quads.size();) {
+    size_t e = i;
+    while (e < quads.size() && quads[e].l == quads[i].l && quads[e].m == quads[i].m) e++;
+    const size_t half = (e - i + 1) / 2;  // n and n + half together, so that neighbours read neighbours
+    for (size_t j = 0; j < half; j++) {
+      const Quad& a = quads[i + j];
+      const bool two = i + j + half < e;
+      const Quad& b = two ? quads[i + j + half] : a;
+      KOctet o;
+      o.l = (short)a.l;
+      o.m = (short)a.m;
+      o.n[0] = (short)a.n;
+      o.n[1] = (short)b.n;
+      for (int t = 0; t < 4; t++) {
+        o.k[t] = a.k[t];
+        o.k[4 + t] = two ? b.k[t] : -1;
+      }
+      out.push_back(o);
+    }
+    i = e;
+  }
 }
 
 double recip_energy_from_parts(const DevSystem& S, const double* host_parts) {

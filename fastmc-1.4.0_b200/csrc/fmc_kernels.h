@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "fmc_device.cuh"
 
 namespace fmc {
@@ -92,9 +94,26 @@ cudaError_t launch_commit(int K, double2* sk, const double2* sk_new, const Commi
                           cudaStream_t st);
 size_t recip_scratch_doubles(const DevSystem& S, int natoms);
 int recip_nparts(const DevSystem& S);
-// Full S(k) of `natoms` atoms {x,y,z,q} into sk; per-block sums of akk|S|^2 into parts.
-cudaError_t launch_recip_full(const DevSystem& S, const double4* atoms, int natoms, double2* sk, double* scratch,
-                              double* parts, cudaStream_t st);
+// Atoms {x,y,z,q} in up to five pieces, taken one after another: piece g from index begin[g] on.
+struct AtomSegs {
+  const double4* p[kMaxGuestTypes + 1];
+  int begin[kMaxGuestTypes + 2];
+  AtomSegs() {
+    for (auto& q : p) q = nullptr;
+    for (int& b : begin) b = 0;
+  }
+  void add(int g, const double4* q, int n) {
+    p[g] = q;
+    for (int i = g + 1; i < kMaxGuestTypes + 2; i++) begin[i] = begin[g] + n;
+  }
+  int total() const { return begin[kMaxGuestTypes + 1]; }
+};
+// Full S(k) of the atoms into sk; per-block sums of akk|S|^2 into parts (recip_nparts of them, device
+// or pinned host memory).
+cudaError_t launch_recip_full(const DevSystem& S, const AtomSegs& atoms, double2* sk, double* scratch, double* parts,
+                              cudaStream_t st);
+// DevSystem::koct of a packed k-vector table.
+void recip_octets(const int* kpacked, int K, std::vector<KOctet>& out);
 double recip_energy_from_parts(const DevSystem& S, const double* host_parts);
 cudaError_t launch_single_point_rs(const DevSystem& S, const GuestView& G, int nsites, const int* sites, const int* lo,
                                    const int* hi, double* out, cudaStream_t st);

@@ -564,7 +564,7 @@ class Server {
     const double per_vox = std::min((double)h.nf, h.nf * (4.0 / 3.0 * kPi * lim * lim * lim) / h.cell.volm);
     const double nv = (double)h.nvox[0] * h.nvox[1] * h.nvox[2];
     double b = 1.15 * nv * per_vox * (sizeof(double4) + 1) + 4.0 * (nv + 1) + 36.0 * h.nf;
-    b += 28.0 * (h.erc.size() + h.vvv.size()) + 4.0 * h.pair_row.size() + 60.0 * h.K;
+    b += 28.0 * (h.erc.size() + h.vvv.size()) + 4.0 * h.pair_row.size() + 100.0 * h.K;
     b += 36.0 * h.deck.maxguest * h.deck.guests.size();
     b += 2.0 * 8.0 * ((double)kSampleCap * h.deck.guests.size() + 1);  // stored production samples
     return (size_t)b + (64u << 10);

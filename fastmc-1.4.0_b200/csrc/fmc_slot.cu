@@ -62,7 +62,7 @@ size_t al(size_t n) { return (n + 255) & ~size_t(255); }
 
 // Host arrays of a system in the order they are staged, with their byte sizes.
 struct Parts {
-  size_t fw, ftype, erc, vvv, prow, kp, akk;
+  size_t fw, ftype, erc, vvv, prow, kp, oct, akk;
   explicit Parts(const HostSystem& h)
       : fw(sizeof(double4) * h.nf),
         ftype(sizeof(int) * h.nf),
@@ -70,9 +70,10 @@ struct Parts {
         vvv(sizeof(double) * h.vvv.size()),
         prow(sizeof(int) * h.pair_row.size()),
         kp(sizeof(int) * h.K),
+        oct(sizeof(KOctet) * h.K),  // at most one a k-vector
         akk(sizeof(double) * h.K) {}
   size_t total() const {
-    return al(fw) + al(ftype) + al(erc) + al(vvv) + al(prow) + al(kp) + al(akk);
+    return al(fw) + al(ftype) + al(erc) + al(vvv) + al(prow) + al(kp) + al(oct) + al(akk);
   }
 };
 
@@ -160,7 +161,7 @@ int build_slot(const HostSystem& h, int slot, const int seed[4], SlotMemory& mem
     return at;
   };
   const size_t o_fw = place(P.fw), o_ft = place(P.ftype), o_erc = place(P.erc), o_vvv = place(P.vvv),
-               o_prow = place(P.prow), o_kp = place(P.kp),
+               o_prow = place(P.prow), o_kp = place(P.kp), o_oct = place(P.oct),
                o_akk = place(P.akk);
   {
     double4* fw = (double4*)(hs + o_fw);
@@ -171,6 +172,10 @@ int build_slot(const HostSystem& h, int slot, const int seed[4], SlotMemory& mem
     std::memcpy(hs + o_prow, h.pair_row.data(), P.prow);
     int* kp = (int*)(hs + o_kp);
     for (int k = 0; k < h.K; k++) kp[k] = kpack(h.kl[k], h.km[k], h.kn[k]);
+    std::vector<KOctet> oct;
+    recip_octets(kp, h.K, oct);
+    v.noct = (int)oct.size();
+    std::memcpy(hs + o_oct, oct.data(), sizeof(KOctet) * oct.size());
     std::memcpy(hs + o_akk, h.akk.data(), P.akk);
   }
   unsigned char* d = nullptr;
@@ -205,6 +210,7 @@ int build_slot(const HostSystem& h, int slot, const int seed[4], SlotMemory& mem
   v.vvv = (const double*)(d + o_vvv);
   v.pair_row = (const int*)(d + o_prow);
   v.kpack = (const int*)(d + o_kp);
+  v.koct = (const KOctet*)(d + o_oct);
   v.akk = (const double*)(d + o_akk);
   for (int a = 0; a < 3; a++) v.nvox[a] = h.nvox[a];
   // voxel lists: count, device prefix sum, fill up to the capacity
@@ -241,7 +247,11 @@ int build_slot(const HostSystem& h, int slot, const int seed[4], SlotMemory& mem
   if ((e = mem.alloc((void**)&skfw, sizeof(double2) * std::max(h.K, 1))) != cudaSuccess) goto fail;
   e = mem.alloc((void**)&scratch, sizeof(double) * std::max<size_t>(recip_scratch_doubles(v, h.nf), 1));
   if (e == cudaSuccess) e = mem.alloc((void**)&parts, sizeof(double) * (recip_nparts(v) + 1));
-  if (e == cudaSuccess) e = launch_recip_full(v, v.fw, h.nf, skfw, scratch, parts, st);
+  if (e == cudaSuccess) {
+    AtomSegs atoms;
+    atoms.add(0, v.fw, h.nf);
+    e = launch_recip_full(v, atoms, skfw, scratch, parts, st);
+  }
   if (e != cudaSuccess) goto fail;
   {
     int ts = 0;
