@@ -167,6 +167,7 @@ int fmc_ewald1_guest(fmc_chain* c, int iguest, int natms, const double* xyz, int
   A.nnew = A.move == fmc::kDelete ? 0 : natms;
   A.ex_lo = A.ex_hi = -1;
   A.engsic = C.sys.engsic[iguest];
+  A.seq = C.pass_seq += 1.0;
   const double* olds = A.move == fmc::kDisplace ? c->pending_old : xyz;
   int w = 0;
   for (int i = 0; i < A.nold; i++, w++) {
@@ -188,7 +189,9 @@ int fmc_ewald1_guest(fmc_chain* c, int iguest, int natms, const double* xyz, int
   cudaError_t e = fmc::launch_pass(C.dsys.view, C.guest_view(), A, C.sk, C.sk_new, C.W, C.st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(C.st);  // the kernel wrote the result to pinned memory
   if (e != cudaSuccess) return fail(-100 - (int)e, cudaGetErrorString(e));
-  out[0] = C.W.result[0];
+  const int over = 1;
+  if (!C.collect(A, &over, out)) return fail(-13, "the pass ended without its results");
+  C.pass_seq_done = C.pass_seq;
   if (A.move == fmc::kDisplace) c->pending_g = -1;
   if (engcpe) *engcpe = out[0];
   return 0;
@@ -220,13 +223,20 @@ int fmc_guest_realspace(fmc_chain* c, int iguest, int natms, const double* xyz, 
     A.q[i] = G.charge[i];
     A.type[i] = (unsigned char)G.type[i];
   }
+  A.single = natms == 1;
+  A.seq = C.pass_seq += 1.0;
+  C.place_sites(A);
   if (int rc0 = C.stop_server()) return fail(rc0, "the resident pass kernel did not end");
   C.take_pending(A);  // an update left by fmc_commit is read through and written by this pass
   cudaError_t e = fmc::launch_pass(C.dsys.view, C.guest_view(), A, C.sk, C.sk_new, C.W, C.st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(C.st);  // the kernel wrote the result to pinned memory
   if (e != cudaSuccess) return fail(-100 - (int)e, cudaGetErrorString(e));
-  if (ewld2) *ewld2 = C.W.result[1];
-  if (vdw) *vdw = C.W.result[2];
+  const int over = 1;
+  double out[3];
+  if (!C.collect(A, &over, out)) return fail(-13, "the pass ended without its results");
+  C.pass_seq_done = C.pass_seq;
+  if (ewld2) *ewld2 = out[1];
+  if (vdw) *vdw = out[2];
   return 0;
 }
 

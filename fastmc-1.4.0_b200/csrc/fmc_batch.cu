@@ -716,14 +716,6 @@ __device__ __forceinline__ double2 recip_term(int k, int nsite, int k1, int k2, 
   return make_double2(ak[k], fma(-so.y, so.y, fma(-so.x, so.x, fma(sw.x, sw.x, sw.y * sw.y))));
 }
 
-constexpr double kMagic = 6755399441055744.0;  // 1.5 x 2^52: adding it rounds to an integer
-
-// How a chunk's pairs are imaged and tabulated, compiled separately so that the loop holds one form
-// (each copy costs instruction cache): orthorhombic cells (imcon 1, 2) and parallelepipeds (3) with
-// one table spacing, and everything else (half-shift cells, slabs, rvdw other than rcut) reading the
-// boundary condition from the cell.
-enum PairKind : int { kPairOrtho = 0, kPairTriclinic = 1, kPairGeneral = 2 };
-
 // One candidate of a chunk: its atom and type (-1: none in this lane), and the trial site the chunk
 // belongs to (the same for every lane).
 struct Cand {
@@ -774,12 +766,6 @@ __device__ __forceinline__ void load_chunk(const BatchSmem& B, int chunk, int nc
   }
 }
 
-// x - nint(x) (halves away from zero) by the rounding of an addition.
-__device__ __forceinline__ double nint_rest(double x) {
-  const double f = x - ((x + kMagic) - kMagic);
-  return fabs(f) == 0.5 ? copysign(0.5, -x) : f;
-}
-
 // This warp's share of the real-space pairs (ewald2 + srfrce over guestlistgen's set): chunks warp,
 // warp + NW, ... of the work list, each lane adding its pairs in that order.  The loop is bound by
 // latency (two chains, 16 warps, share an SM): a pair is a candidate load, an image, a root, three
@@ -800,9 +786,7 @@ __device__ __forceinline__ void real_space(const BatchSmem& B, double& v1, doubl
   };
   const int at0 = begins(lane), at1 = begins(lane + 32);
   const int nminus = M.nnew ? nold : 0;  // a displacement's old sites are subtracted
-  const double rcut2 = S.rcut2, rdr = S.rdr_e;
-  // imcon 1 takes the first edge for every axis (images, utility_pack.f:1138-1349)
-  const int iy = S.cell.imcon == 1 ? 0 : 1, iz = S.cell.imcon == 1 ? 0 : 2;
+  const double rcut2 = S.rcut2;
   Cand c[U];
 #pragma unroll
   for (int u = 0; u < U; u++) {
@@ -818,27 +802,7 @@ __device__ __forceinline__ void real_space(const BatchSmem& B, double& v1, doubl
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const int s = c[u].site;
-      double dx = M.x[s] - c[u].x, dy = M.y[s] - c[u].y, dz = M.z[s] - c[u].z;
-      if (KIND == kPairOrtho) {
-        // nint by the rounding of an addition: a tie picks either image, at the same distance
-        const double* hh = S.cell.h;
-        const double* ri = S.cell.inv;
-        dx = fma(-hh[0], fma(ri[0], dx, kMagic) - kMagic, dx);
-        dy = fma(-hh[4 * iy], fma(ri[iy], dy, kMagic) - kMagic, dy);
-        dz = fma(-hh[4 * iz], fma(ri[iz], dz, kMagic) - kMagic, dz);
-      } else if (KIND == kPairTriclinic) {
-        const double* r = S.cell.rh;
-        const double* hh = S.cell.h;
-        const double fx = nint_rest(r[0] * dx + r[3] * dy + r[6] * dz);
-        const double fy = nint_rest(r[1] * dx + r[4] * dy + r[7] * dz);
-        const double fz = nint_rest(r[2] * dx + r[5] * dy + r[8] * dz);
-        dx = hh[0] * fx + hh[3] * fy + hh[6] * fz;
-        dy = hh[1] * fx + hh[4] * fy + hh[7] * fz;
-        dz = hh[2] * fx + hh[5] * fy + hh[8] * fz;
-      } else {
-        min_image(S.cell, dx, dy, dz);
-      }
-      const double rsq = fma(dx, dx, fma(dy, dy, dz * dz));
+      const double rsq = image_dist2<KIND>(S.cell, M.x[s] - c[u].x, M.y[s] - c[u].y, M.z[s] - c[u].z);
       const bool in = c[u].type >= 0 && rsq < rcut2;
       const double qq = M.cq[s] * c[u].q;
       rs[u] = in ? rsq : rcut2;
@@ -850,23 +814,7 @@ __device__ __forceinline__ void real_space(const BatchSmem& B, double& v1, doubl
     for (int u = 0; u < U; u++) load_chunk(B, base + (U + u) * NW, nchunk, nsite, at0, at1, c[u]);
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      const double sg = site[u] < nminus ? -1.0 : 1.0;
-      const double r = sqrt_approx(rs[u]);
-      const double x = __dmul_rn(r, rdr);
-      const double f = (x - 0.5) + kMagic;  // floor(x) but for integers, where either interval agrees
-      const int l = __double2loint(f);
-      const double p = x - (f - kMagic), pm = p - 1.0, hp = 0.5 * p;
-      if (KIND != kPairGeneral) {
-        const double2* tb = S.pair_tab + (off[u] + l);
-        const double2 a0 = tb[0], a1 = tb[1], a2 = tb[2];
-        const double e1 = fma(a1.x - a0.x, p, a0.x), e2 = fma(a2.x - a1.x, pm, a1.x);
-        const double w1 = fma(a1.y - a0.y, p, a0.y), w2 = fma(a2.y - a1.y, pm, a1.y);
-        v1 = fma(fma(e2 - e1, hp, e1), cq[u], v1);
-        v2 = fma(fma(w2 - w1, hp, w1), sg, v2);
-      } else {
-        v1 = fma(interp3(S.erc, r, rdr), cq[u], v1);
-        if (off[u]) v2 = fma(interp3(S.vvv + off[u], r, S.rdr_v), sg, v2);
-      }
+      pair_table<KIND>(S, rs[u], cq[u], off[u], site[u] < nminus ? -1.0 : 1.0, v1, v2);
     }
   }
 }
@@ -977,9 +925,9 @@ __device__ __noinline__ void sums_kind(int kmax_smem, int stride) {
 
 template <int NT, int KPT, int CPT>
 __device__ __forceinline__ void sums(const DevSystem& S, int kmax_smem, int stride) {
-  const int imcon = S.cell.imcon;
-  if (S.pair_tab && imcon <= 2) sums_kind<kPairOrtho, NT, KPT, CPT>(kmax_smem, stride);
-  else if (S.pair_tab && imcon == 3) sums_kind<kPairTriclinic, NT, KPT, CPT>(kmax_smem, stride);
+  const int kind = pair_kind(S);
+  if (kind == kPairOrtho) sums_kind<kPairOrtho, NT, KPT, CPT>(kmax_smem, stride);
+  else if (kind == kPairTriclinic) sums_kind<kPairTriclinic, NT, KPT, CPT>(kmax_smem, stride);
   else sums_kind<kPairGeneral, NT, KPT, CPT>(kmax_smem, stride);
 }
 

@@ -77,6 +77,7 @@ int upload_system(const HostSystem& h, DeviceSystem& d, std::string& err) {
       goto fail;
     }
     for (int i = 0; i < nv; i++) offv[i + 1] = offv[i] + cnt[i];
+    d.vox_off = offv;
     const size_t ne = (size_t)offv[nv];
     d.vox_entries = (long long)ne;
     int* atoms = nullptr;
@@ -182,11 +183,11 @@ Chain::~Chain() {
     if (srv_words) cudaFreeHost(srv_words);
     if (d_fl) cudaFree(d_fl);
     cudaStreamSynchronize(st);
-    for (void* p : {(void*)sk, (void*)sk_new, (void*)sk_save, (void*)gsite, (void*)gtype, (void*)W.recip_part, (void*)W.site_e,
-                    (void*)W.counter, (void*)recip_scratch, (void*)sp_work})
+    for (void* p : {(void*)sk, (void*)sk_new, (void*)sk_save, (void*)gsite, (void*)gtype, (void*)W.counter, (void*)recip_scratch})
       if (p) cudaFree(p);
     if (recip_parts) cudaFreeHost(recip_parts);
-    if (W.result) cudaFreeHost(W.result);
+    if (sp_work) cudaFreeHost(sp_work);
+    if (W.slots) cudaFreeHost(W.slots);
     cudaStreamDestroy(st);
   }
 }
@@ -264,13 +265,14 @@ int Chain::open_prepared(HostSystem&& prepared, const int seed[4], int dev, std:
   FMC_CUDA(cudaMalloc(&gtype, sizeof(int) * std::max(gcap, 1)));
   W.gsite = gsite;
   W.gtype = gtype;
-  FMC_CUDA(cudaMalloc(&W.recip_part, sizeof(double) * (pass_recip_blocks(dsys.view) + 1)));
-  FMC_CUDA(cudaMalloc(&W.site_e, sizeof(double) * 2 * kMaxPassSites));
   FMC_CUDA(cudaMalloc(&W.counter, sizeof(unsigned)));
   FMC_CUDA(cudaMemset(W.counter, 0, sizeof(unsigned)));
-  // the pass result goes straight to pinned host memory, which the kernel addresses through unified
+  // the blocks' energies go straight to pinned host memory, which the kernel addresses through unified
   // addressing: a copy back per pass cost as much as a third of the plain path's time
-  FMC_CUDA(cudaMallocHost(&W.result, sizeof(double) * 4));
+  W.recip_slots = (pass_recip_blocks(dsys.view) + 1) & ~1;
+  const size_t slot_words = 2 * (size_t)W.recip_slots + 4 * kMaxPassSites;
+  FMC_CUDA(cudaMallocHost(&W.slots, sizeof(double) * slot_words));
+  std::memset(W.slots, 0, sizeof(double) * slot_words);
   FMC_CUDA(cudaStreamCreateWithFlags(&srv_st, cudaStreamNonBlocking));
   FMC_CUDA(cudaMallocHost(&mb, sizeof(PassMailbox)));
   FMC_CUDA(cudaMallocHost(&h_fl, sizeof(PassServerFlags)));
@@ -464,37 +466,23 @@ int Chain::single_point() {
   double ewald1eng = 0, e2 = 0, ev = 0, e3 = 0;
   if (nguest_sites > 0) {
     ewald1eng = eall - ewald1sum;
-    // one entry per guest site: its index and its own molecule's site range
-    std::vector<int> idx, lo, hi;
-    for (int g = 0; g < (int)sp.size(); g++)
-      for (int m = 0; m < sp[g].nmol; m++)
-        for (int i = 0; i < sp[g].nsite; i++) {
-          idx.push_back(sp[g].seg_off + m * sp[g].nsite + i);
-          lo.push_back(sp[g].seg_off + m * sp[g].nsite);
-          hi.push_back(sp[g].seg_off + (m + 1) * sp[g].nsite);
-        }
-    const int n = (int)idx.size();
-    // workspace of the chain's own, grown when the guests need more of it
-    const size_t need = sizeof(double) * 4 * n + sizeof(int) * 3 * n;
-    if (need > sp_cap) {
-      if (sp_work) cudaFree(sp_work);
+    const int n = nguest_sites;
+    int nsite[kMaxGuestTypes] = {};
+    for (int g = 0; g < (int)sp.size(); g++) nsite[g] = sp[g].nsite;
+    // workspace of the chain's own in pinned memory, which the kernel writes: grown when the guests
+    // need more of it
+    if ((size_t)n > sp_cap) {
+      if (sp_work) cudaFreeHost(sp_work);
       sp_work = nullptr;
       sp_cap = 0;
-      e = cudaMalloc(&sp_work, need + need / 2);
-      if (e == cudaSuccess) sp_cap = need + need / 2;
+      const size_t cap = (size_t)n + n / 2;
+      e = cudaMallocHost(&sp_work, sizeof(double) * 4 * cap);
+      if (e == cudaSuccess) sp_cap = cap;
     }
-    double* dout = sp_work;
-    int* dbuf = reinterpret_cast<int*>(sp_work + 4 * (size_t)n);
-    std::vector<int> packed;
-    packed.insert(packed.end(), idx.begin(), idx.end());
-    packed.insert(packed.end(), lo.begin(), lo.end());
-    packed.insert(packed.end(), hi.begin(), hi.end());
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dbuf, packed.data(), sizeof(int) * 3 * n, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = launch_single_point_rs(dsys.view, guest_view(), n, dbuf, dbuf + n, dbuf + 2 * n, dout, st);
-    std::vector<double> out(4 * n);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out.data(), dout, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = launch_single_point_rs(dsys.view, guest_view(), nsite, sp_work, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return sync_error(e);
+    const double* out = sp_work;
     double cf = 0, vf = 0, cg = 0, vg = 0;
     for (int i = 0; i < n; i++) {
       cf += out[4 * i];
@@ -593,6 +581,8 @@ int Chain::pass_resident(const PassArgs& A, double out[3]) {
     B.z[i] = A.z[i];
     B.q[i] = A.q[i];
     B.type[i] = A.type[i];
+    B.vb[i] = A.vb[i];
+    B.vl[i] = A.vl[i];
   }
   B.pc = A.pc;
   mb->G = guest_view();
@@ -600,30 +590,74 @@ int Chain::pass_resident(const PassArgs& A, double out[3]) {
   mb->sk_new = sk_new;
   std::atomic_thread_fence(std::memory_order_release);
   *(volatile long long*)&mb->cmd = (long long)A.seq;
-  volatile double* flag = W.result + 3;
   for (int restarts = 0;;) {
-    long long spins = 0;
-    while (*flag != A.seq && !*(volatile int*)&srv_words[0] && ++spins < 400000000LL) {
-    }
-    std::atomic_thread_fence(std::memory_order_acquire);
-    if (*flag == A.seq) break;
+    if (collect(A, &srv_words[0], out)) break;
     // the kernel ended without the pass, or nothing came back in time: end it, start it again
     *(volatile int*)&mb->quit = 1;
     cudaError_t e = cudaStreamSynchronize(srv_st);
     srv_live = false;
     *(volatile int*)&mb->quit = 0;
     if (e != cudaSuccess) return sync_error(e);
-    if (*flag == A.seq) break;
+    const int over = 1;
+    if (collect(A, &over, out)) break;
     if (srv_words[1] || ++restarts > 3) return -13;  // a wait inside the kernel ran out
     int rc = start_server();
     if (rc) return rc;
     if (!srv_live) return -13;
   }
-  out[0] = W.result[0];
-  out[1] = W.result[1];
-  out[2] = W.result[2];
   srv_passes++;
   return 0;
+}
+
+void Chain::place_sites(PassArgs& A) const {
+  const DevSystem& S = dsys.view;
+  for (int i = 0; i < A.nold + A.nnew; i++) {
+    const int v = voxel_of(S, A.x[i], A.y[i], A.z[i]);
+    A.vb[i] = dsys.vox_off[v];
+    A.vl[i] = dsys.vox_off[v + 1] - dsys.vox_off[v];
+  }
+}
+
+// The words of one block's slot, once their stamp is that of pass seq.
+static bool slot_arrived(const double* p, double seq, int n, double* out) {
+  const volatile double* v = p;
+  const double stamp = v[n];
+  double e[2] = {v[0], n > 1 ? v[1] : 0.0};
+  const double want = pass_stamp(seq, e[0], e[1]);
+  if (std::memcmp(&stamp, &want, sizeof(stamp))) return false;
+  std::copy(e, e + n, out);
+  return true;
+}
+
+bool Chain::collect(const PassArgs& A, const volatile int* ended, double out[3]) const {
+  // block by block, in the order in which they are added; the wait for all of them is bounded (well over
+  // a second)
+  long long spins = 0;
+  auto wait = [&](const double* p, int n, double* e) {
+    while (!slot_arrived(p, A.seq, n, e)) {
+      if (ended && *ended) return slot_arrived(p, A.seq, n, e);
+      if (++spins >= 400000000LL) return false;
+    }
+    return true;
+  };
+  double r = 0.0, e2 = 0.0, ev = 0.0, e[2];
+  for (int b = 0; b < A.nbk; b++) {
+    if (!wait(W.recip_slot(b), 1, e)) return false;
+    r += e[0];
+  }
+  for (int s = 0; A.do_real && s < A.nold + A.nnew; s++) {
+    if (!wait(W.site_slot(s), 2, e)) return false;
+    const bool minus = s < A.nold && A.move == kDisplace;
+    e2 = minus ? e2 - e[0] : e2 + e[0];
+    ev = minus ? ev - e[1] : ev + e[1];
+  }
+  double ewld1 = dsys.view.recip_pref * r;
+  if (A.move == kInsert) ewld1 = ewld1 + A.engsic;
+  if (A.move == kDelete) ewld1 = ewld1 - A.engsic;
+  out[0] = ewld1;
+  out[1] = e2;
+  out[2] = ev;
+  return true;
 }
 
 int Chain::pass(int move, int g, int mol, const double* old_xyz, const double* new_xyz, double out[3]) {
@@ -642,6 +676,7 @@ int Chain::pass(int move, int g, int mol, const double* old_xyz, const double* n
     A.ex_hi = A.ex_lo + s.nsite;
   }
   A.engsic = sys.engsic[g];
+  A.single = s.nsite == 1;
   int w = 0;
   for (int i = 0; i < A.nold; i++, w++) {
     A.x[w] = old_xyz[3 * i];
@@ -657,6 +692,7 @@ int Chain::pass(int move, int g, int mol, const double* old_xyz, const double* n
     A.q[w] = G.charge[i];
     A.type[w] = (unsigned char)G.type[i];
   }
+  place_sites(A);
   if (profile && !ev0) {
     cudaEventCreate(&ev0);
     cudaEventCreate(&ev1);
@@ -680,19 +716,12 @@ int Chain::pass(int move, int g, int mol, const double* old_xyz, const double* n
   }
   cudaError_t e = launch_pass(dsys.view, guest_view(), A, sk, sk_new, W, st);
   if (profile) cudaEventRecord(ev1, st);
-  if (e == cudaSuccess && !profile) {
-    // the kernel writes its energies and then this pass's sequence number into pinned host memory;
-    // waiting for the number is quicker than synchronising the stream.  The wait is bounded (well
-    // over a second), after which the stream is synchronised, which also reports a failed kernel.
-    volatile double* flag = W.result + 3;
-    long long spins = 0;
-    while (*flag != pass_seq && ++spins < 400000000LL) {
-    }
-    // the energies were written before the number: read them only after the number (acquire)
-    std::atomic_thread_fence(std::memory_order_acquire);
-    if (*flag != pass_seq) e = cudaStreamSynchronize(st);
-  } else if (e == cudaSuccess) {
-    e = cudaStreamSynchronize(st);  // profiled passes: the events need the stream
+  if (e == cudaSuccess && (profile || !collect(A, nullptr, out))) {
+    // profiled passes: the events need the stream; otherwise nothing came in time, and synchronising also
+    // reports a failed kernel
+    e = cudaStreamSynchronize(st);
+    const int over = 1;
+    if (e == cudaSuccess && !collect(A, &over, out)) return -13;  // the kernel ended without its results
   }
   if (e != cudaSuccess) return sync_error(e);
   if (profile) {
@@ -701,9 +730,6 @@ int Chain::pass(int move, int g, int mol, const double* old_xyz, const double* n
     pass_ms += ms;
     pass_timed++;
   }
-  out[0] = W.result[0];
-  out[1] = W.result[1];
-  out[2] = W.result[2];
   passes++;
   pass_seq_done = pass_seq;
   return 0;

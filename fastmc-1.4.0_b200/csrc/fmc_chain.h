@@ -24,6 +24,7 @@ struct DeviceSystem {
   std::vector<void*> allocations;
   int device = 0;
   long long vox_entries = 0;
+  std::vector<int> vox_off;  // host copy of the voxel lists' offsets
   ~DeviceSystem();
 };
 
@@ -56,7 +57,7 @@ class Chain {
   double* recip_scratch = nullptr;
   double* recip_parts = nullptr;  // pinned
   size_t recip_scratch_n = 0;
-  double* sp_work = nullptr;  // single-point workspace, grown when a call needs more
+  double* sp_work = nullptr;  // single-point workspace (pinned, 4 doubles a guest site), grown as needed
   size_t sp_cap = 0;
   // host mirror
   std::vector<Species> sp;
@@ -83,7 +84,7 @@ class Chain {
   double despre = 0, presrate = 0;
   // launch accounting and optional CUDA-event timing of the pass kernel
   long long passes = 0, commits = 0;
-  double pass_seq = 0.0;  // sequence number the pass kernel echoes next to its energies
+  double pass_seq = 0.0;  // number of the last pass, stamped next to its energies
   bool profile = false;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double pass_ms = 0.0;
@@ -106,6 +107,12 @@ class Chain {
   // left pending for the next pass to read through and write (no launch of its own); a second
   // update before the next pass, or one of more than kMaxPendSites sites, is written at once.
   int commit(int move, int g, int mol, const double* new_xyz);
+  // The voxel lists of a pass's sites, found on the host: the kernel reads their entries at once.
+  void place_sites(PassArgs& A) const;
+  // Waits for the blocks of a launched pass and adds their energies up in block order into out =
+  // {ewld1, ewld2, vdw}; false when they do not come in time, or *ended (if given) says that the kernel
+  // ended and they are not there.
+  bool collect(const PassArgs& A, const volatile int* ended, double out[3]) const;
   // Hands the pending guest-site update to a pass about to launch (or marks none).
   void take_pending(PassArgs& A);
   // Writes the pending guest-site update now (before anything else reads the device sites).

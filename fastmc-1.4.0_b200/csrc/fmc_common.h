@@ -83,6 +83,22 @@ FMC_HD double duni_next(Duni& d) {
   return (double)uni;
 }
 
+// The stamp beside a block's energies a, b in pinned memory: the pass's number folded with their bits, so
+// that a reader knows the words belong to pass `seq` in whatever order they arrived.  (Compared as
+// words: a double of any bits.)
+FMC_HD double pass_stamp(double seq, double a, double b) {
+  union {
+    double d;
+    unsigned long long u;
+  } s, x, y;
+  s.d = seq;
+  x.d = a;
+  y.d = b;
+  s.u *= 0x9E3779B97F4A7C15ULL;  // spreads the few bits in which two passes' numbers differ
+  s.u ^= (x.u << 7 | x.u >> 57) ^ (y.u << 23 | y.u >> 41);
+  return s.d;
+}
+
 // ------------------------------------------------------------------ cell geometry
 struct CellGeom {
   double h[9];    // cell vectors a,b,c (cell(1..9) of the reference, a = h[0..2])

@@ -101,7 +101,7 @@ __device__ __forceinline__ double sqrt_approx(double x) {
 }
 
 // Fractional coordinates s = rcell . r as in ewald.f:106-108.
-__device__ __forceinline__ void frac_coords(const CellGeom& c, double x, double y, double z, double* s) {
+FMC_HD void frac_coords(const CellGeom& c, double x, double y, double z, double* s) {
   const double* r = c.rh;
   s[0] = r[0] * x + r[3] * y + r[6] * z;
   s[1] = r[1] * x + r[4] * y + r[7] * z;
@@ -124,9 +124,74 @@ __device__ __forceinline__ void pair_energy(const DevSystem& S, double dx, doubl
   }
 }
 
+// ------------------------------------------------------------------ pairs without branches
+// How pairs are imaged and tabulated, each compiled by itself: orthorhombic cells (imcon 1, 2) and
+// parallelepipeds (3) whose erc and vvv share one spacing, and everything else (half-shift cells, slabs,
+// rvdw other than rcut) reading the boundary condition from the cell.
+enum PairKind : int { kPairOrtho = 0, kPairTriclinic = 1, kPairGeneral = 2 };
+
+FMC_HD int pair_kind(const DevSystem& S) {
+  return !S.pair_tab || S.cell.imcon > 3 ? kPairGeneral : (S.cell.imcon == 3 ? kPairTriclinic : kPairOrtho);
+}
+
+constexpr double kMagic = 6755399441055744.0;  // 1.5 x 2^52: adding it rounds to an integer
+
+// x - nint(x) (halves away from zero) by the rounding of an addition.
+__device__ __forceinline__ double nint_rest(double x) {
+  const double f = x - ((x + kMagic) - kMagic);
+  return fabs(f) == 0.5 ? copysign(0.5, -x) : f;
+}
+
+// Squared distance of the reference's image of a separation (images, utility_pack.f:1138-1349).
+template <int KIND>
+__device__ __forceinline__ double image_dist2(const CellGeom& c, double dx, double dy, double dz) {
+  if (KIND == kPairOrtho) {
+    // nint by the rounding of an addition: a tie picks either image, at the same distance; imcon 1
+    // takes the first edge for every axis
+    const int iy = c.imcon == 1 ? 0 : 1, iz = c.imcon == 1 ? 0 : 2;
+    dx = fma(-c.h[0], fma(c.inv[0], dx, kMagic) - kMagic, dx);
+    dy = fma(-c.h[4 * iy], fma(c.inv[iy], dy, kMagic) - kMagic, dy);
+    dz = fma(-c.h[4 * iz], fma(c.inv[iz], dz, kMagic) - kMagic, dz);
+  } else if (KIND == kPairTriclinic) {
+    const double *r = c.rh, *h = c.h;
+    const double fx = nint_rest(r[0] * dx + r[3] * dy + r[6] * dz);
+    const double fy = nint_rest(r[1] * dx + r[4] * dy + r[7] * dz);
+    const double fz = nint_rest(r[2] * dx + r[5] * dy + r[8] * dz);
+    dx = h[0] * fx + h[3] * fy + h[6] * fz;
+    dy = h[1] * fx + h[4] * fy + h[7] * fz;
+    dz = h[2] * fx + h[5] * fy + h[8] * fz;
+  } else {
+    min_image(c, dx, dy, dz);
+  }
+  return fma(dx, dx, fma(dy, dy, dz * dz));
+}
+
+// Adds a pair's table energies: v1 += cq erc(r), v2 += sg vvv(r) with r^2 = rs <= rcut^2 and the row that
+// begins at `off` (0: none; row 0 of the interleaved table holds no vdW).
+template <int KIND>
+__device__ __forceinline__ void pair_table(const DevSystem& S, double rs, double cq, int off, double sg, double& v1,
+                                           double& v2) {
+  const double r = sqrt_approx(rs);
+  const double x = __dmul_rn(r, S.rdr_e);
+  const double f = (x - 0.5) + kMagic;  // floor(x) but for integers, where either interval agrees
+  const int l = __double2loint(f);
+  const double p = x - (f - kMagic), pm = p - 1.0, hp = 0.5 * p;
+  if (KIND != kPairGeneral) {
+    const double2* tb = S.pair_tab + (off + l);
+    const double2 a0 = tb[0], a1 = tb[1], a2 = tb[2];
+    const double e1 = fma(a1.x - a0.x, p, a0.x), e2 = fma(a2.x - a1.x, pm, a1.x);
+    const double w1 = fma(a1.y - a0.y, p, a0.y), w2 = fma(a2.y - a1.y, pm, a1.y);
+    v1 = fma(fma(e2 - e1, hp, e1), cq, v1);
+    v2 = fma(fma(w2 - w1, hp, w1), sg, v2);
+  } else {
+    v1 = fma(interp3(S.erc, r, S.rdr_e), cq, v1);
+    if (off) v2 = fma(interp3(S.vvv + off, r, S.rdr_v), sg, v2);
+  }
+}
+
 // Voxel of a position (wrapped into the cell; a slab's z clamped to its layers, whose lowest and
 // highest hold no atom).
-__device__ __forceinline__ int voxel_of(const DevSystem& S, double x, double y, double z) {
+FMC_HD int voxel_of(const DevSystem& S, double x, double y, double z) {
   double s[3];
   if (S.cell.imcon == 6) {
     const CellGeom& c = S.cell;
@@ -168,9 +233,12 @@ struct PendingCommit {
 
 // Thread-partial real-space energy of one site against the framework (voxel list) and the
 // guest sites outside [ex_lo, ex_hi).  Threads stride by `nthr` starting at `tid`.
+//
+// Single-site molecules only (pass_block): their moves without an energy change are decided by what
+// these sums round off, so they keep this arithmetic and order.
 __device__ __forceinline__ void site_partial(const DevSystem& S, const GuestView& G, const PendingCommit& P, double px,
-                                             double py, double pz, double q, int ty, int ex_lo, int ex_hi, int tid,
-                                             int nthr, double& ec_fw, double& ev_fw, double& ec_g, double& ev_g) {
+                                             double py, double pz, double q, int ty, int vb, int vl, int ex_lo,
+                                             int ex_hi, int tid, int nthr, double& ec_fw, double& ev_fw, double& ec_g, double& ev_g) {
   const double chgea = q * kR4pie0;
   const int* prow = S.pair_row + ty * (S.ntypes + 1);
   for (int sg = 0; sg < G.nseg; sg++) {
@@ -195,11 +263,90 @@ __device__ __forceinline__ void site_partial(const DevSystem& S, const GuestView
       pair_energy(S, px - a.x, py - a.y, pz - a.z, chgea, a.w, prow[t], ec_g, ev_g);
     }
   }
-  int v = voxel_of(S, px, py, pz);
-  int b = S.vox_off[v], e = S.vox_off[v + 1];
+  const int b = vb, e = vb + vl;
   for (int i = b + tid; i < e; i += nthr) {
     double4 a = S.vox_xyzq[i];
     pair_energy(S, px - a.x, py - a.y, pz - a.z, chgea, a.w, prow[S.vox_type[i]], ec_fw, ev_fw);
+  }
+}
+
+// The guest site j of segment sg as if the pending update were written.
+__device__ __forceinline__ void guest_site(const GuestView& G, const PendingCommit& P, int sg, int j, double4& a,
+                                           int& t) {
+  if (sg == P.seg && j >= P.lo) {
+    if (P.op == kDelete) {  // the sites after the removed molecule, one molecule on
+      j += P.ns;
+    } else if (j < P.lo + P.ns) {  // the inserted or displaced molecule
+      a = P.site[j - P.lo];
+      t = P.type[j - P.lo];
+      return;
+    }
+  }
+  a = G.site[j];
+  t = G.type[j];
+}
+
+// A thread's share of the pairs of one site with n candidates: two candidates in flight, distances
+// first, then the tables, without a branch between (a lane whose candidate is missing or beyond the
+// cut-off reads row 0 at the cut-off and adds zero).  fetch(i, atom, type) gives candidate i, leaving
+// type at -1 for one to skip; prow: the table row's offset for each type, there once every thread has
+// called ready(), which happens after the first candidates are on their way.
+template <int KIND, class Fetch, class Ready>
+__device__ __forceinline__ void pair_sum(const DevSystem& S, const int* prow, double px, double py, double pz,
+                                         double chgea, int n, int tid, int nthr, Fetch fetch, Ready ready, double& ec,
+                                         double& ev) {
+  constexpr int U = 2;
+  bool first = true;
+  int base = tid;
+  do {
+    double4 a[U];
+    int t[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      a[u] = make_double4(0.0, 0.0, 0.0, 0.0);
+      t[u] = -1;
+      if (base + u * nthr < n) fetch(base + u * nthr, a[u], t[u]);
+    }
+    if (first) ready();
+    first = false;
+    double rs[U], cq[U];
+    int off[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const double rsq = image_dist2<KIND>(S.cell, px - a[u].x, py - a[u].y, pz - a[u].z);
+      const bool in = t[u] >= 0 && rsq < S.rcut2;
+      const double qq = chgea * a[u].w;
+      rs[u] = in ? rsq : S.rcut2;
+      cq[u] = in && fabs(qq) > 1e-10 ? qq : 0.0;  // ewald2 skips smaller products
+      off[u] = in ? prow[t[u]] : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) pair_table<KIND>(S, rs[u], cq[u], off[u], 1.0, ec, ev);
+    base += U * nthr;
+  } while (base < n);
+}
+
+// A thread's share of one site's real-space energy against the framework (the voxel list of vl entries
+// from vb) and the guest sites outside [ex_lo, ex_hi).
+template <int KIND, class Ready>
+__device__ __forceinline__ void site_pairs(const DevSystem& S, const GuestView& G, const PendingCommit& P,
+                                           const int* prow, double px, double py, double pz, double q, int vb, int vl,
+                                           int ex_lo, int ex_hi, int tid, int nthr, Ready ready, double& ec_fw,
+                                           double& ev_fw, double& ec_g, double& ev_g) {
+  const double chgea = q * kR4pie0;
+  pair_sum<KIND>(S, prow, px, py, pz, chgea, vl, tid, nthr,
+                 [&](int i, double4& a, int& t) {
+                   a = S.vox_xyzq[vb + i];
+                   t = S.vox_type[vb + i];
+                 },
+                 ready, ec_fw, ev_fw);
+  for (int sg = 0; sg < G.nseg; sg++) {
+    const int lo = G.seg_off[sg];
+    pair_sum<KIND>(S, prow, px, py, pz, chgea, G.seg_len[sg], tid, nthr,
+                   [&](int i, double4& a, int& t) {
+                     if (lo + i < ex_lo || lo + i >= ex_hi) guest_site(G, P, sg, lo + i, a, t);
+                   },
+                   [] {}, ec_g, ev_g);
   }
 }
 

@@ -15,6 +15,7 @@
 #include <cmath>
 #include <cstddef>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "fmc_device.cuh"
@@ -23,7 +24,6 @@
 namespace fmc {
 
 constexpr int kPassThreads = 256;
-static_assert(2 * kMaxPassSites <= kPassThreads, "the combine stages every site energy in one pass");
 
 // A guest-site update by one block (all its threads): a delete removes [lo, lo+ns) and shifts
 // the rest of the segment down in order; an insert writes at the segment end, a displacement
@@ -55,15 +55,34 @@ __device__ __forceinline__ void apply_commit(const PendingCommit& P, double4* si
 }
 
 // ------------------------------------------------------------------------------ pass
+struct PassSmem {
+  double red[32 * 2];
+  int prow[256];  // the vdW row's offset of the block's site with each type (at most 255 types)
+  bool am_last;
+};
+
+// A word pair to pinned memory in one store.
+__device__ __forceinline__ void publish(double* p, double a, double b) {
+  asm volatile("st.volatile.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(a), "d"(b) : "memory");
+}
+
 // One block's share of a trial pass (block `blk` of `nblocks`): blocks [0, nbk) the reciprocal
-// change of 256 k-vectors each, the next nsite blocks the real-space energy of one trial site
-// each (further blocks idle), then the last block to finish combines the partials in a fixed
-// order into {ewld1, ewld2, vdw}, publishes them with the sequence number and writes the pending
-// guest-site update.  Returns (to every thread) whether this block was the last.
+// change of 256 k-vectors each, the next nsite blocks the real-space energy of one trial site each
+// (further blocks idle).  Each writes its energy, stamped with the pass's number, to its own words of
+// pinned memory, from which the host adds them up in order.  Where a guest-site update is pending
+// (or `ticket` asks for it) the last block to finish then writes the update, every block having read
+// the sites.  Returns (to every thread) whether this block was the last of a counted pass.
+//
+// A pass is one trial of one chain, some twenty blocks: it lasts as long as its chain of dependent reads.
+// So what a block needs is read as early as its address is known -- the host finds each site's voxel
+// list, a reciprocal block reads its k-vectors before it builds the phases, a real-space block its first
+// candidates before the row offsets are there -- and nothing is combined on the device: a ticket with
+// its fences took 0.8 us, reading the partials back and ordering the result behind them 1.2 us, of a
+// kernel of 5 us (3,392 atoms, K = 4192); the stamp says on its own that a block's words have arrived.
 template <class Args>
 __device__ __forceinline__ bool pass_block(const DevSystem& S, const GuestView& G, const Args& A, const double2* sk,
                                            double2* sk_new, const PassScratch& W, int blk, int nblocks,
-                                           double2* sm_tab, double* red, double* comb, bool& am_last) {
+                                           double2* sm_tab, PassSmem& sm, bool ticket) {
   const int nsite = A.nold + A.nnew;
   const int nbk = A.nbk;
   const int tid = threadIdx.x;
@@ -71,6 +90,15 @@ __device__ __forceinline__ bool pass_block(const DevSystem& S, const GuestView& 
     // ---- reciprocal space
     const int k1 = S.kmax[0], k2 = S.kmax[1], k3 = S.kmax[2];
     const int stride = (k1 + 1) + (k2 + 1) + (k3 + 1);
+    const int k = blk * blockDim.x + tid;
+    int kp = 0;
+    double2 so = make_double2(0.0, 0.0);
+    double ak = 0.0;
+    if (k < S.K) {
+      kp = S.kpack[k];
+      so = sk[k];
+      ak = S.akk[k];
+    }
     for (int w = tid; w < nsite * 3; w += blockDim.x) {
       int s = w / 3, ax = w % 3;
       double f[3];
@@ -80,12 +108,12 @@ __device__ __forceinline__ bool pass_block(const DevSystem& S, const GuestView& 
     }
     __syncthreads();
     double v[1] = {0.0};
-    int k = blk * blockDim.x + tid;
     if (k < S.K) {
       int l, m, n;
-      kunpack(S.kpack[k], l, m, n);
+      kunpack(kp, l, m, n);
       int am = m < 0 ? -m : m, an = n < 0 ? -n : n;
       double2 aold = make_double2(0.0, 0.0), anew = make_double2(0.0, 0.0);
+#pragma unroll 3
       for (int s = 0; s < nsite; s++) {
         const double2* t = sm_tab + s * stride;
         double2 e1 = t[l], e2 = t[k1 + 1 + am], e3 = t[k1 + k2 + 2 + an];
@@ -100,7 +128,7 @@ __device__ __forceinline__ bool pass_block(const DevSystem& S, const GuestView& 
           anew.y += q * c.y;
         }
       }
-      double2 so = sk[k], sn;
+      double2 sn;
       if (A.move == kInsert)
         sn = make_double2(anew.x + so.x, anew.y + so.y);
       else if (A.move == kDelete)
@@ -108,82 +136,63 @@ __device__ __forceinline__ bool pass_block(const DevSystem& S, const GuestView& 
       else
         sn = make_double2((so.x - aold.x) + anew.x, (so.y - aold.y) + anew.y);
       sk_new[k] = sn;
-      v[0] = S.akk[k] * (sn.x * sn.x + sn.y * sn.y - so.x * so.x - so.y * so.y);
+      v[0] = ak * (sn.x * sn.x + sn.y * sn.y - so.x * so.x - so.y * so.y);
     }
-    block_sum<1>(v, red);
-    if (tid == 0) W.recip_part[blk] = v[0];
+    block_sum<1>(v, sm.red);
+    if (tid == 0) publish(W.recip_slot(blk), v[0], pass_stamp(A.seq, v[0], 0.0));
   } else if (A.do_real && blk - nbk < nsite) {
     // ---- real space of one trial site
     const int s = blk - nbk;
     double v[2] = {0.0, 0.0};
     double ec_fw = 0.0, ev_fw = 0.0, ec_g = 0.0, ev_g = 0.0;
-    site_partial(S, G, A.pc, A.x[s], A.y[s], A.z[s], A.q[s], A.type[s], A.ex_lo, A.ex_hi, tid, blockDim.x, ec_fw,
-                 ev_fw, ec_g, ev_g);
+    if (A.single) {
+      site_partial(S, G, A.pc, A.x[s], A.y[s], A.z[s], A.q[s], A.type[s], A.vb[s], A.vl[s], A.ex_lo, A.ex_hi, tid,
+                   blockDim.x, ec_fw, ev_fw, ec_g, ev_g);
+    } else {
+      const int row = tid <= S.ntypes ? max(S.pair_row[A.type[s] * (S.ntypes + 1) + tid], 0) * S.tab_stride : 0;
+      auto rows = [&]() {
+        if (tid <= S.ntypes) sm.prow[tid] = row;
+        __syncthreads();
+      };
+      const int kind = pair_kind(S);
+      auto pairs = [&](auto k) {
+        site_pairs<decltype(k)::value>(S, G, A.pc, sm.prow, A.x[s], A.y[s], A.z[s], A.q[s], A.vb[s], A.vl[s], A.ex_lo,
+                                       A.ex_hi, tid, blockDim.x, rows, ec_fw, ev_fw, ec_g, ev_g);
+      };
+      if (kind == kPairOrtho) pairs(std::integral_constant<int, kPairOrtho>());
+      else if (kind == kPairTriclinic) pairs(std::integral_constant<int, kPairTriclinic>());
+      else pairs(std::integral_constant<int, kPairGeneral>());
+    }
     v[0] = ec_g + ec_fw;
     v[1] = ev_g + ev_fw;
-    block_sum<2>(v, red);
+    block_sum<2>(v, sm.red);
     if (tid == 0) {
-      W.site_e[2 * s] = v[0];
-      W.site_e[2 * s + 1] = v[1];
+      publish(W.site_slot(s), v[0], v[1]);
+      publish(W.site_slot(s) + 2, pass_stamp(A.seq, v[0], v[1]), 0.0);
     }
   }
-  // ---- last block combines in a fixed order: the partials are loaded by all its threads at
-  // once and summed by thread 0 in block / site order
+  if (!ticket && !A.pc.op) return false;
   if (tid == 0) {
-    __threadfence();
-    unsigned done = atomicAdd(W.counter, 1u);
-    am_last = (done == (unsigned)nblocks - 1);
+    // every thread's reads and writes of this pass come before the count (block_sum's barriers, or no
+    // work at all), the update after it
+    unsigned done;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(done) : "l"(W.counter) : "memory");
+    sm.am_last = done == (unsigned)nblocks - 1;
+    if (sm.am_last) *W.counter = 0u;
   }
   __syncthreads();
-  if (!am_last) return false;
-  __threadfence();
-  double r = 0.0;
-  for (int base = 0; base < nbk; base += kPassThreads) {
-    if (base + tid < nbk) comb[tid] = ((volatile double*)W.recip_part)[base + tid];
-    __syncthreads();
-    if (tid == 0)
-      for (int i = 0; i < kPassThreads && base + i < nbk; i++) r += comb[i];
-    __syncthreads();
-  }
-  const int nse = A.do_real ? 2 * nsite : 0;  // <= 2 * kMaxPassSites <= kPassThreads
-  if (tid < nse) comb[tid] = ((volatile double*)W.site_e)[tid];
-  __syncthreads();
-  if (tid == 0) {
-    double ewld1 = S.recip_pref * r;
-    if (A.move == kInsert) ewld1 = ewld1 + A.engsic;
-    if (A.move == kDelete) ewld1 = ewld1 - A.engsic;
-    double e2 = 0.0, ev = 0.0;
-    const double* se = comb;
-    for (int s = 0; s < (A.do_real ? nsite : 0); s++) {
-      if (s < A.nold && A.move == kDisplace) {
-        e2 = e2 - se[2 * s];
-        ev = ev - se[2 * s + 1];
-      } else {
-        e2 = e2 + se[2 * s];
-        ev = ev + se[2 * s + 1];
-      }
-    }
-    W.result[0] = ewld1;
-    W.result[1] = e2;
-    W.result[2] = ev;
-    __threadfence_system();  // the energies reach the host before the sequence number does
-    ((volatile double*)W.result)[3] = A.seq;
-    *W.counter = 0u;
-  }
-  // every block has read the guest sites: the last one writes the pending update
+  if (!sm.am_last) return false;
   if (A.pc.op) apply_commit(A.pc, W.gsite, W.gtype);
   return true;
 }
 
 template <int N>
-__global__ void __launch_bounds__(kPassThreads) fmc_pass_kernel(DevSystem S, GuestView G, PassArgsT<N> A,
+__global__ void __launch_bounds__(kPassThreads, 1) fmc_pass_kernel(DevSystem S, GuestView G, PassArgsT<N> A,
                                                                 const double2* __restrict__ sk, double2* sk_new,
                                                                 PassScratch W) {
   extern __shared__ double2 sm_tab[];
-  __shared__ double red[32 * 2];
-  __shared__ double comb[kPassThreads];
-  __shared__ bool am_last;
-  pass_block(S, G, A, sk, sk_new, W, (int)blockIdx.x, (int)gridDim.x, sm_tab, red, comb, am_last);
+  __shared__ PassSmem sm;
+  pass_block(S, G, A, sk, sk_new, W, (int)blockIdx.x, (int)gridDim.x, sm_tab, sm, false);
 }
 
 // ------------------------------------------------------------------------------ resident pass
@@ -204,9 +213,7 @@ __global__ void __launch_bounds__(kPassThreads) fmc_pass_server_kernel(DevSystem
                                                                        PassScratch W, long long seq0,
                                                                        long long idle_ns) {
   extern __shared__ double2 sm_tab[];
-  __shared__ double red[32 * 2];
-  __shared__ double comb[kPassThreads];
-  __shared__ bool am_last;
+  __shared__ PassSmem sm;
   __shared__ long long s_cmd;
   __shared__ PassArgsT<kSmallPassSites> A;
   __shared__ GuestView G;
@@ -294,8 +301,8 @@ __global__ void __launch_bounds__(kPassThreads) fmc_pass_server_kernel(DevSystem
       __syncthreads();
       if (tid == 0) *(volatile unsigned long long*)&fl->go = (unsigned long long)c;
     }
-    const bool last = pass_block(S, G, A, s_sk, s_sk_new, W, (int)blockIdx.x, (int)gridDim.x, sm_tab, red, comb,
-                                 am_last);
+    const bool last = pass_block(S, G, A, s_sk, s_sk_new, W, (int)blockIdx.x, (int)gridDim.x, sm_tab, sm,
+                                 true);
     if (last) {
       __syncthreads();  // the update is written by every thread of this block
       if (tid == 0) {
@@ -350,6 +357,8 @@ cudaError_t launch_pass(const DevSystem& S, const GuestView& G, const PassArgs& 
       B.z[i] = A.z[i];
       B.q[i] = A.q[i];
       B.type[i] = A.type[i];
+      B.vb[i] = A.vb[i];
+      B.vl[i] = A.vl[i];
     }
     B.pc = A.pc;
     fmc_pass_kernel<kSmallPassSites><<<grid, kPassThreads, smem, st>>>(S, G, B, sk, sk_new, W);
@@ -668,28 +677,48 @@ double recip_energy_from_parts(const DevSystem& S, const double* host_parts) {
 }
 
 // ------------------------------------------------------------------------------ single point
-// For entry b: site i = sites[b]; out[4*b + {0,1,2,3}] = {coulomb vs framework, vdw vs
-// framework, coulomb vs other guests, vdw vs other guests}; own molecule = [lo[b], hi[b]).
-__global__ void fmc_sp_kernel(DevSystem S, GuestView G, const int* __restrict__ sites, const int* __restrict__ lo,
-                              const int* __restrict__ hi, double* out) {
+// Block b: guest site b of the segments in order; out[4*b + {0,1,2,3}] = {coulomb vs framework, vdw vs
+// framework, coulomb vs other guests, vdw vs other guests}.
+struct MolSites {
+  int n[kMaxGuestTypes];  // sites per molecule of each species
+};
+
+template <int KIND>
+__global__ void __launch_bounds__(256, 2) fmc_sp_kernel(DevSystem S, GuestView G, MolSites mol, double* out) {
   __shared__ double red[32 * 4];
-  const int b = blockIdx.x, i = sites[b];
-  double4 a = G.site[i];
-  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  __shared__ int prow[256];
+  int r = blockIdx.x, sg = 0;
+  while (r >= G.seg_len[sg]) r -= G.seg_len[sg++];
+  const int i = G.seg_off[sg] + r, lo = G.seg_off[sg] + r / mol.n[sg] * mol.n[sg], hi = lo + mol.n[sg];
+  const double4 a = G.site[i];
+  if ((int)threadIdx.x <= S.ntypes)
+    prow[threadIdx.x] = max(S.pair_row[G.type[i] * (S.ntypes + 1) + threadIdx.x], 0) * S.tab_stride;
+  const int v = voxel_of(S, a.x, a.y, a.z), vb = S.vox_off[v], vl = S.vox_off[v + 1] - vb;
   PendingCommit none;
   none.op = 0;
   none.seg = -1;
   none.lo = none.ns = none.seg_end = 0;
-  site_partial(S, G, none, a.x, a.y, a.z, a.w, G.type[i], lo[b], hi[b], threadIdx.x, blockDim.x, v[0], v[1], v[2],
-               v[3]);
-  block_sum<4>(v, red);
+  double e[4] = {0.0, 0.0, 0.0, 0.0};
+  site_pairs<KIND>(S, G, none, prow, a.x, a.y, a.z, a.w, vb, vl, lo, hi, threadIdx.x, blockDim.x,
+                   [] { __syncthreads(); }, e[0], e[1], e[2], e[3]);
+  block_sum<4>(e, red);
   if (threadIdx.x == 0)
-    for (int k = 0; k < 4; k++) out[4 * b + k] = v[k];
+    for (int k = 0; k < 4; k++) out[4 * blockIdx.x + k] = e[k];
 }
 
-cudaError_t launch_single_point_rs(const DevSystem& S, const GuestView& G, int nsites, const int* sites, const int* lo,
-                                   const int* hi, double* out, cudaStream_t st) {
-  if (nsites > 0) fmc_sp_kernel<<<nsites, 256, 0, st>>>(S, G, sites, lo, hi, out);
+cudaError_t launch_single_point_rs(const DevSystem& S, const GuestView& G, const int* nsite, double* out,
+                                   cudaStream_t st) {
+  MolSites mol;
+  int n = 0;
+  for (int g = 0; g < kMaxGuestTypes; g++) {
+    mol.n[g] = g < G.nseg ? nsite[g] : 1;
+    if (g < G.nseg) n += G.seg_len[g];
+  }
+  if (n == 0) return cudaSuccess;
+  const int kind = pair_kind(S);
+  if (kind == kPairOrtho) fmc_sp_kernel<kPairOrtho><<<n, 256, 0, st>>>(S, G, mol, out);
+  else if (kind == kPairTriclinic) fmc_sp_kernel<kPairTriclinic><<<n, 256, 0, st>>>(S, G, mol, out);
+  else fmc_sp_kernel<kPairGeneral><<<n, 256, 0, st>>>(S, G, mol, out);
   return cudaGetLastError();
 }
 

@@ -21,9 +21,11 @@ struct PassArgsT {
   int do_real;        // 1: one real-space block per site
   int nold, nnew;
   int ex_lo, ex_hi;   // guest-site range of the moving molecule (excluded from real space)
+  int single, pad;    // a single-site molecule: real space in its fixed order (site_partial)
   double engsic;      // self-interaction term of the species (ewald.f:87-93)
-  double seq;         // copied to result[3] after the energies, for a host that polls (0: none)
+  double seq;         // the pass's number, which stamps its results (pass_stamp)
   double x[N], y[N], z[N], q[N];
+  int vb[N], vl[N];   // each site's voxel list: first entry, length (do_real)
   unsigned char type[N];
   PendingCommit pc;   // an accepted guest-site update this pass reads through and then writes
 };
@@ -32,10 +34,13 @@ using PassArgs = PassArgsT<kMaxPassSites>;
 
 // Scratch of one pass launch (global memory beyond inputs and outputs).
 struct PassScratch {
-  double* recip_part;  // [ceil(K/256)]
-  double* site_e;      // [2*kMaxPassSites]
   unsigned* counter;   // last-block ticket, left at zero by the kernel
-  double* result;      // {ewld1, ewld2, vdw, seq} in pinned host memory, written by the kernel directly
+  // pinned host memory, written by the kernel directly: per reciprocal block {sum akk d|S|^2, stamp}, then
+  // (32-byte aligned) per site {ewld2, vdw, stamp, -}
+  double* slots;
+  int recip_slots;     // room for reciprocal blocks, even
+  FMC_HD double* recip_slot(int b) const { return slots + 2 * b; }
+  FMC_HD double* site_slot(int s) const { return slots + 2 * recip_slots + 4 * s; }
   double4* gsite;      // the chain's guest sites and types, written by the last block when the
   int* gtype;          // pass carries a pending update (PassArgs::pc)
 };
@@ -115,8 +120,10 @@ cudaError_t launch_recip_full(const DevSystem& S, const AtomSegs& atoms, double2
 // DevSystem::koct of a packed k-vector table.
 void recip_octets(const int* kpacked, int K, std::vector<KOctet>& out);
 double recip_energy_from_parts(const DevSystem& S, const double* host_parts);
-cudaError_t launch_single_point_rs(const DevSystem& S, const GuestView& G, int nsites, const int* sites, const int* lo,
-                                   const int* hi, double* out, cudaStream_t st);
+// Real-space energies of every guest site present (four doubles each, in segment order; device or
+// pinned host memory); nsite: sites per molecule of each species.
+cudaError_t launch_single_point_rs(const DevSystem& S, const GuestView& G, const int* nsite, double* out,
+                                   cudaStream_t st);
 
 // Voxel lists: per voxel, the framework atoms within sqrt(lim2) of its centre by true minimum
 // image, in ascending atom order.  Orthorhombic cells (voxel_prefilter_applies) can pass
