@@ -178,16 +178,12 @@ Chain::~Chain() {
     cudaSetDevice(device);
     stop_server();
     if (srv_st) cudaStreamDestroy(srv_st);
-    if (mb) cudaFreeHost(mb);
-    if (h_fl) cudaFreeHost(h_fl);
-    if (srv_words) cudaFreeHost(srv_words);
     if (d_fl) cudaFree(d_fl);
     cudaStreamSynchronize(st);
     for (void* p : {(void*)sk, (void*)sk_new, (void*)sk_save, (void*)gsite, (void*)gtype, (void*)W.counter, (void*)recip_scratch})
       if (p) cudaFree(p);
-    if (recip_parts) cudaFreeHost(recip_parts);
     if (sp_work) cudaFreeHost(sp_work);
-    if (W.slots) cudaFreeHost(W.slots);
+    if (pinned) cudaFreeHost(pinned);
     cudaStreamDestroy(st);
   }
 }
@@ -271,19 +267,30 @@ int Chain::open_prepared(HostSystem&& prepared, const int seed[4], int dev, std:
   // addressing: a copy back per pass cost as much as a third of the plain path's time
   W.recip_slots = (pass_recip_blocks(dsys.view) + 1) & ~1;
   const size_t slot_words = 2 * (size_t)W.recip_slots + 4 * kMaxPassSites;
-  FMC_CUDA(cudaMallocHost(&W.slots, sizeof(double) * slot_words));
-  std::memset(W.slots, 0, sizeof(double) * slot_words);
+  // One allocation, each part on 4 KB of its own. The full S(k)'s energy partials (of the framework alone and
+  // of all atoms) are in it too, so that there is no copy back to wait for.
+  size_t bytes = 0;
+  auto part = [&](size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 4095) & ~(size_t)4095;
+    return at;
+  };
+  const size_t at_slots = part(sizeof(double) * slot_words), at_mb = part(sizeof(PassMailbox)),
+               at_fl = part(sizeof(PassServerFlags)), at_words = part(sizeof(int) * 2),
+               at_parts = part(sizeof(double) * 2 * (recip_nparts(dsys.view) + 1)), at_sk = part(sizeof(double2) * K);
+  FMC_CUDA(cudaMallocHost(&pinned, bytes));
+  std::memset(pinned, 0, bytes);
+  char* base = (char*)pinned;
+  W.slots = (double*)(base + at_slots);
+  mb = (PassMailbox*)(base + at_mb);
+  h_fl = (PassServerFlags*)(base + at_fl);
+  srv_words = (int*)(base + at_words);
+  recip_parts = (double*)(base + at_parts);
+  sk_host = (double2*)(base + at_sk);
   FMC_CUDA(cudaStreamCreateWithFlags(&srv_st, cudaStreamNonBlocking));
-  FMC_CUDA(cudaMallocHost(&mb, sizeof(PassMailbox)));
-  FMC_CUDA(cudaMallocHost(&h_fl, sizeof(PassServerFlags)));
-  FMC_CUDA(cudaMallocHost(&srv_words, sizeof(int) * 2));
   FMC_CUDA(cudaMalloc(&d_fl, sizeof(PassServerFlags)));
-  std::memset(mb, 0, sizeof(PassMailbox));
-  srv_words[0] = srv_words[1] = 0;
   recip_scratch_n = recip_scratch_doubles(dsys.view, sys.nf + gcap);
   FMC_CUDA(cudaMalloc(&recip_scratch, sizeof(double) * recip_scratch_n));
-  // energy partials in pinned host memory, written by the kernel: no copy back to wait for
-  FMC_CUDA(cudaMallocHost(&recip_parts, sizeof(double) * (recip_nparts(dsys.view) + 1)));
   // upload preloaded guests
   for (int g = 0; g < ng; g++) {
     rc = set_guests(g, sp[g].nmol, sp[g].xyz.data());
@@ -410,23 +417,31 @@ int Chain::restart(const Revive& r, std::string& err) {
 }
 
 // S(k) over all current atoms: guests in species order, then the framework (condense order).
-int Chain::full_recip(double* e_out) {
-  if (int rc0 = stop_server()) return rc0;  // nothing else runs beside the resident kernel
-  if (int rc = flush_commit()) return rc;
+cudaError_t Chain::queue_recip(double* parts) {
   AtomSegs atoms;
   const int ng = (int)sp.size();
   for (int g = 0; g < ng; g++) atoms.add(g, gsite + sp[g].seg_off, sp[g].nmol * sp[g].nsite);
   atoms.add(ng, dsys.view.fw, sys.nf);
-  cudaError_t e = launch_recip_full(dsys.view, atoms, sk, recip_scratch, recip_parts, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return sync_error(e);
+  return launch_recip_full(dsys.view, atoms, sk, recip_scratch, parts, st);
+}
+
+double Chain::recip_with_self(const double* parts) const {
   double q2 = 0.0;
   for (int g = 0; g < (int)sp.size(); g++)
     for (int m = 0; m < sp[g].nmol; m++)
       for (int i = 0; i < sp[g].nsite; i++) q2 = q2 + sys.deck.guests[g].charge[i] * sys.deck.guests[g].charge[i];
   for (int i = 0; i < sys.nf; i++) q2 = q2 + sys.fq[i] * sys.fq[i];
   double engsic = -kR4pie0 * sys.alpha * q2 / kSqrPi;
-  if (e_out) *e_out = recip_energy_from_parts(dsys.view, recip_parts) + engsic;
+  return recip_energy_from_parts(dsys.view, parts) + engsic;
+}
+
+int Chain::full_recip(double* e_out) {
+  if (int rc0 = stop_server()) return rc0;  // nothing else runs beside the resident kernel
+  if (int rc = flush_commit()) return rc;
+  cudaError_t e = queue_recip(recip_parts);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return sync_error(e);
+  if (e_out) *e_out = recip_with_self(recip_parts);
   return 0;
 }
 
@@ -436,18 +451,14 @@ int Chain::full_recip(double* e_out) {
 int Chain::single_point() {
   if (int rc0 = stop_server()) return rc0;  // nothing else runs beside the resident kernel
   if (int rc = flush_commit()) return rc;
-  // framework only
-  AtomSegs fw;
+  // The three sums are queued together and waited for once, behind the host's own part: a wait after each
+  // left the device idle for a round trip of about 8 us between them.
+  AtomSegs fw;  // framework only
   fw.add(0, dsys.view.fw, sys.nf);
-  cudaError_t e = launch_recip_full(dsys.view, fw, sk, recip_scratch, recip_parts, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  double* fw_parts = recip_parts + recip_nparts(dsys.view) + 1;
+  cudaError_t e = launch_recip_full(dsys.view, fw, sk, recip_scratch, fw_parts, st);
+  if (e == cudaSuccess) e = queue_recip(recip_parts);
   if (e != cudaSuccess) return sync_error(e);
-  double q2f = 0.0;
-  for (int i = 0; i < sys.nf; i++) q2f = q2f + sys.fq[i] * sys.fq[i];
-  ewald1sum = recip_energy_from_parts(dsys.view, recip_parts) + (-kR4pie0 * sys.alpha * q2f / kSqrPi);
-  double eall = 0.0;
-  int rc = full_recip(&eall);
-  if (rc) return rc;
   // numtyp / numfrz over all atoms (lrcorrect, vdw_terms.f:542-553)
   numtyp.assign(sys.ntypes + 1, 0);
   numfrz.assign(sys.ntypes + 1, 0);
@@ -462,11 +473,8 @@ int Chain::single_point() {
         numtyp[sys.deck.guests[g].type[i]]++;
         nguest_sites++;
       }
-  double elrc0 = lrc_energy(sys, numtyp, numfrz);
-  double ewald1eng = 0, e2 = 0, ev = 0, e3 = 0;
-  if (nguest_sites > 0) {
-    ewald1eng = eall - ewald1sum;
-    const int n = nguest_sites;
+  const int n = nguest_sites;
+  if (n > 0) {
     int nsite[kMaxGuestTypes] = {};
     for (int g = 0; g < (int)sp.size(); g++) nsite[g] = sp[g].nsite;
     // workspace of the chain's own in pinned memory, which the kernel writes: grown when the guests
@@ -480,18 +488,10 @@ int Chain::single_point() {
       if (e == cudaSuccess) sp_cap = cap;
     }
     if (e == cudaSuccess) e = launch_single_point_rs(dsys.view, guest_view(), nsite, sp_work, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return sync_error(e);
-    const double* out = sp_work;
-    double cf = 0, vf = 0, cg = 0, vg = 0;
-    for (int i = 0; i < n; i++) {
-      cf += out[4 * i];
-      vf += out[4 * i + 1];
-      cg += out[4 * i + 2];
-      vg += out[4 * i + 3];
-    }
-    e2 = cf + 0.5 * cg;
-    ev = vf + 0.5 * vg;
+  }
+  double elrc0 = lrc_energy(sys, numtyp, numfrz);
+  double ewald1eng = 0, e2 = 0, ev = 0, e3 = 0;
+  if (n > 0) {
     // intramolecular exclusion correction from the actual coordinates (ewald3 over the
     // exclusion lists, gcmc.f:2676-2697)
     for (int g = 0; g < (int)sp.size(); g++) {
@@ -510,6 +510,25 @@ int Chain::single_point() {
         }
       }
     }
+  }
+  double q2f = 0.0;
+  for (int i = 0; i < sys.nf; i++) q2f = q2f + sys.fq[i] * sys.fq[i];
+  const cudaError_t es = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = es;
+  if (e != cudaSuccess) return sync_error(e);
+  ewald1sum = recip_energy_from_parts(dsys.view, fw_parts) + (-kR4pie0 * sys.alpha * q2f / kSqrPi);
+  if (n > 0) {
+    ewald1eng = recip_with_self(recip_parts) - ewald1sum;
+    const double* out = sp_work;
+    double cf = 0, vf = 0, cg = 0, vg = 0;
+    for (int i = 0; i < n; i++) {
+      cf += out[4 * i];
+      vf += out[4 * i + 1];
+      cg += out[4 * i + 2];
+      vg += out[4 * i + 3];
+    }
+    e2 = cf + 0.5 * cg;
+    ev = vf + 0.5 * vg;
     double ecoulg = ewald1eng + e2 + e3, evdwg = ev + elrc0;
     spenergy = (ecoulg + evdwg) / sys.engunit;
   } else {

@@ -55,7 +55,9 @@ class Chain {
   int gcap = 0;
   PassScratch W{};
   double* recip_scratch = nullptr;
-  double* recip_parts = nullptr;  // pinned
+  double* recip_parts = nullptr;  // pinned: all atoms' energy partials, then the framework's
+  double2* sk_host = nullptr;     // pinned staging of S(k) for a caller
+  void* pinned = nullptr;         // the chain's pinned memory: pass slots, mailbox, flags and the two above
   size_t recip_scratch_n = 0;
   double* sp_work = nullptr;  // single-point workspace (pinned, 4 doubles a guest site), grown as needed
   size_t sp_cap = 0;
@@ -135,6 +137,8 @@ class Chain {
   int start_server();
   int stop_server();
   int pass_resident(const PassArgs& A, double out[3]);
+  cudaError_t queue_recip(double* parts);     // launches S(k) of all current atoms; energy partials to parts
+  double recip_with_self(const double* parts) const;
   int full_recip(double* e_recip_plus_self);  // S(k) over all current atoms (ewald1)
   int single_point();
   int step(MoveRecord* rec);
