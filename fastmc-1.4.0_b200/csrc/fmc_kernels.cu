@@ -757,156 +757,178 @@ __device__ __forceinline__ void voxel_centre(const CellGeom& c, int v, int n0, i
   p[2] = fa * c.h[2] + fb * c.h[5] + fc * c.h[8];
 }
 
+// A warp builds the lists of two consecutive voxels (one where a distance takes up to 27 images), 32 atoms
+// at a time: no barriers, and an atom is read once for all of them.  In orthorhombic cells (imcon 1, 2) a distance is taken in float first, which decides all but the atoms within `margin` of the limit; those few
+// are measured in double, so that the lists hold exactly the atoms of the double test.  The margin, with h
+// the longest period and s the largest |atom| + |centre| + h of an axis: rounding the coordinates, their
+// difference and n periods moves a separation by at most 3 * 2^-24 s and its square by h times that; where
+// it picks the other of two images, the square moves by at most 2^-21 h s.  Three axes: 2.2e-6 h s in all,
+// half of the margin.
+// Bound by instructions issued (a test is some 20, and 3 for the atom's conversions) and, in the fill, by
+// stores of the two or so of 32 atoms that are in a list.  5,928 atoms and 28,656 lists: count 238 us, fill 560
+// us, against 517 and 1,112 with a block a voxel, a prefilter by voxel and four barriers every 128 atoms;
+// 424 atoms: 28 us for both against 30.  Four voxels a warp: 250 and 523 us, but 34 us for 424 atoms; eight:
+// 226 and 608, 41.
 constexpr int kVoxThreads = 128;
 
-// Voxel prefilter of orthorhombic cells (imcon 1, 2).  code[j] packs atom j's voxel along
-// a, b, c (10 bits each); an atom whose voxel lies more than reach voxels away (cyclically)
-// along any axis from the list's voxel cannot be within the list radius, so the list kernels
-// skip its FP64 distance test.  reach = floor((lim + 0.01 A) / edge + 1.5): half a voxel for
-// the atom's place inside its voxel, one for an atom binned into a neighbouring voxel by
-// rounding, 0.01 A for rounding of the distance test itself and of the periods.  The lists
-// keep exactly the atoms, and the order, of the unfiltered test.
-__device__ __forceinline__ int cyclic_gap(int d, int n) {
-  d = d < 0 ? -d : d;
-  return min(d, n - d);
-}
+template <bool kOrtho>
+constexpr int kVoxPerWarp = kOrtho ? 2 : 1;
 
-__device__ __forceinline__ bool voxel_near(unsigned cd, int va, int vb, int vc, int n0, int n1, int n2, int3 r) {
-  return cyclic_gap(va - (int)(cd & 1023u), n0) <= r.x && cyclic_gap(vb - (int)((cd >> 10) & 1023u), n1) <= r.y &&
-         cyclic_gap(vc - (int)(cd >> 20), n2) <= r.z;
-}
+struct VoxelCell {  // an orthorhombic cell's side of the float test, converted on the host: conversions are slow
+  float h[3], r[3], lim, scale;  // scale: 4.4e-6 h
+};
 
-__global__ void __launch_bounds__(kVoxThreads) fmc_voxel_code_kernel(CellGeom cell, int n0, int n1, int n2,
-                                                                     const double4* __restrict__ fw, int nf,
-                                                                     unsigned* __restrict__ code) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nf) return;
-  const double4 a = fw[j];
-  const double x[3] = {a.x, a.y, a.z};
-  const int n[3] = {n0, n1, n2};
-  unsigned out = 0;
-  for (int k = 0; k < 3; k++) {
-    double f = x[k] / cell.h[4 * k];
-    f -= floor(f);
-    const int i = min(max((int)(f * n[k]), 0), n[k] - 1);
-    out |= (unsigned)i << (10 * k);
-  }
-  code[j] = out;
-}
-
-__global__ void __launch_bounds__(kVoxThreads) fmc_voxel_count_kernel(CellGeom cell, int n0, int n1, int n2,
-                                                                      const double4* __restrict__ fw, int nf,
-                                                                      double lim2, const unsigned* __restrict__ code,
-                                                                      int3 reach, int* counts) {
-  __shared__ int ws[kVoxThreads / 32];
+struct VoxelCentre {
+  float x, y, z, lo, hi;  // lo, hi: the limit less and plus the margin's part that is not the atom's
   double p[3];
-  voxel_centre(cell, blockIdx.x, n0, n1, n2, p);
-  const int va = blockIdx.x / (n1 * n2), vb = (blockIdx.x / n2) % n1, vc = blockIdx.x % n2;
-  int cnt = 0;
-  for (int j = threadIdx.x; j < nf; j += blockDim.x) {
-    if (code && !voxel_near(code[j], va, vb, vc, n0, n1, n2, reach)) continue;
-    double4 a = fw[j];
-    if (true_dist2_dev(cell, p[0] - a.x, p[1] - a.y, p[2] - a.z) < lim2) cnt++;
+};
+
+// Flags, for each of the warp's voxels, of this lane's atom (live: there is one).
+template <bool kOrtho>
+__device__ __forceinline__ void voxel_flags(const CellGeom& c, const VoxelCell& f, const double4& a, bool live,
+                                            double lim2, const VoxelCentre* t, bool* flag) {
+  constexpr int V = kVoxPerWarp<kOrtho>;
+  bool open[V], some = false;
+  if (kOrtho) {
+    constexpr float kRound = 12582912.0f;  // 1.5 * 2^23: adding it rounds to the nearest integer
+    const float ax = (float)a.x, ay = (float)a.y, az = (float)a.z;
+    const float margin = f.scale * fmaxf(fabsf(ax), fmaxf(fabsf(ay), fabsf(az)));
+#pragma unroll
+    for (int u = 0; u < V; u++) {
+      float dx = t[u].x - ax, dy = t[u].y - ay, dz = t[u].z - az;
+      dx = fmaf(-f.h[0], fmaf(f.r[0], dx, kRound) - kRound, dx);
+      dy = fmaf(-f.h[1], fmaf(f.r[1], dy, kRound) - kRound, dy);
+      dz = fmaf(-f.h[2], fmaf(f.r[2], dz, kRound) - kRound, dz);
+      const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+      flag[u] = live && d2 < t[u].lo - margin;
+      open[u] = live && !flag[u] && !(d2 > t[u].hi + margin);
+      some = some || open[u];
+    }
+    if (!__any_sync(0xffffffffu, some)) return;
+  } else {
+#pragma unroll
+    for (int u = 0; u < V; u++) {
+      flag[u] = false;
+      open[u] = live;
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = cnt;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int w = 0; w < kVoxThreads / 32; w++) t += ws[w];
-    counts[blockIdx.x] = t;
-  }
+#pragma unroll
+  for (int u = 0; u < V; u++)
+    if (open[u]) {
+      double dx = t[u].p[0] - a.x, dy = t[u].p[1] - a.y, dz = t[u].p[2] - a.z;
+      if (kOrtho) {  // true_dist2_dev without its other cells: a quarter of the code
+        if (c.imcon == 1) min_image_t<1>(c, dx, dy, dz);
+        else min_image_t<2>(c, dx, dy, dz);
+        flag[u] = dx * dx + dy * dy + dz * dz < lim2;
+      } else {
+        flag[u] = true_dist2_dev(c, dx, dy, dz) < lim2;
+      }
+    }
 }
 
-__global__ void __launch_bounds__(kVoxThreads) fmc_voxel_fill_kernel(CellGeom cell, int n0, int n1, int n2,
-                                                                     const double4* __restrict__ fw,
-                                                                     const int* __restrict__ ftype, int nf, double lim2,
-                                                                     const unsigned* __restrict__ code, int3 reach,
-                                                                     const int* __restrict__ off, int* atoms,
-                                                                     unsigned short* atoms16, double4* xyzq,
-                                                                     unsigned char* vtype, long long cap) {
-  __shared__ int woff[kVoxThreads / 32 + 1];
-  __shared__ int running;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double p[3];
-  voxel_centre(cell, blockIdx.x, n0, n1, n2, p);
-  const int va = blockIdx.x / (n1 * n2), vb = (blockIdx.x / n2) % n1, vc = blockIdx.x % n2;
-  if (threadIdx.x == 0) running = 0;
-  const int base = off[blockIdx.x];
-  __syncthreads();
-  for (int chunk = 0; chunk < nf; chunk += blockDim.x) {
-    int j = chunk + threadIdx.x;
-    bool flag = false;
-    double4 a = make_double4(0, 0, 0, 0);
-    if (j < nf && (!code || voxel_near(code[j], va, vb, vc, n0, n1, n2, reach))) {
-      a = fw[j];
-      flag = true_dist2_dev(cell, p[0] - a.x, p[1] - a.y, p[2] - a.z) < lim2;
+// The lists' lengths (counts), or the lists themselves at off.
+template <bool kOrtho, bool kFill>
+__global__ void __launch_bounds__(kVoxThreads) fmc_voxel_kernel(CellGeom cell, VoxelCell f, int n0, int n1, int n2,
+                                                                const double4* __restrict__ fw,
+                                                                const int* __restrict__ ftype, int nf, double lim2,
+                                                                int* __restrict__ counts, const int* __restrict__ off,
+                                                                int* __restrict__ atoms,
+                                                                unsigned short* __restrict__ atoms16,
+                                                                double4* __restrict__ xyzq,
+                                                                unsigned char* __restrict__ vtype, long long cap) {
+  constexpr int V = kVoxPerWarp<kOrtho>;
+  const int lane = threadIdx.x & 31, nv = n0 * n1 * n2;
+  const int v0 = (blockIdx.x * (kVoxThreads / 32) + (threadIdx.x >> 5)) * V;
+  if (v0 >= nv || nf < 1) return;
+  VoxelCentre t[V];
+  int at[V], end[V];
+#pragma unroll
+  for (int u = 0; u < V; u++) {
+    const int v = min(v0 + u, nv - 1);
+    voxel_centre(cell, v, n0, n1, n2, t[u].p);
+    t[u].x = (float)t[u].p[0];
+    t[u].y = (float)t[u].p[1];
+    t[u].z = (float)t[u].p[2];
+    const float h = fmaxf(f.h[0], fmaxf(f.h[1], f.h[2]));
+    const float margin = f.scale * (h + fmaxf(fabsf(t[u].x), fmaxf(fabsf(t[u].y), fabsf(t[u].z))));
+    t[u].lo = f.lim - margin;
+    t[u].hi = f.lim + margin;
+    at[u] = kFill ? off[v] : 0;
+    // beyond the capacity: the caller compares off[nv] with cap and rebuilds
+    end[u] = kFill && v0 + u < nv ? (int)min((long long)off[v + 1], cap) : 0;
+  }
+  double4 a = fw[min(lane, nf - 1)], next = a;
+#pragma unroll 1
+  for (int base = 0; base < nf; base += 32, a = next) {
+    const int j = base + lane;
+    const bool live = j < nf;
+    next = fw[min(j + 32, nf - 1)];
+    bool flag[V];
+    voxel_flags<kOrtho>(cell, f, a, live, lim2, t, flag);
+    if (!kFill) {
+#pragma unroll
+      for (int u = 0; u < V; u++) at[u] += flag[u];
+      continue;
     }
-    unsigned mask = __ballot_sync(0xffffffffu, flag);
-    if (lane == 0) woff[warp + 1] = __popc(mask);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      woff[0] = 0;
-      for (int w = 1; w <= kVoxThreads / 32; w++) woff[w] += woff[w - 1];
-    }
-    __syncthreads();
-    if (flag) {
-      int pos = base + running + woff[warp] + __popc(mask & ((1u << lane) - 1u));
-      if (pos < cap) {  // beyond the capacity: the caller compares off[nv] with cap and rebuilds
+    const int type = ftype[min(j, nf - 1)];
+#pragma unroll
+    for (int u = 0; u < V; u++) {
+      const unsigned mask = __ballot_sync(0xffffffffu, flag[u]);
+      const int pos = at[u] + __popc(mask & ((1u << lane) - 1u));
+      at[u] += __popc(mask);
+      if (flag[u] && pos < end[u]) {
         if (atoms) atoms[pos] = j;
         if (atoms16) atoms16[pos] = (unsigned short)j;
         xyzq[pos] = a;
-        vtype[pos] = (unsigned char)ftype[j];
+        vtype[pos] = (unsigned char)type;
       }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) running += woff[kVoxThreads / 32];
-    __syncthreads();
   }
+  if (!kFill)
+#pragma unroll
+    for (int u = 0; u < V; u++) {
+      const int n = __reduce_add_sync(0xffffffffu, at[u]);
+      if (lane == 0 && v0 + u < nv) counts[v0 + u] = n;
+    }
 }
 
 namespace {
-int3 voxel_reach(const CellGeom& cell, const int* nvox, double lim2) {
-  const double lim = std::sqrt(lim2) + 0.01;
-  int r[3];
-  for (int a = 0; a < 3; a++) r[a] = (int)std::floor(lim / (cell.h[4 * a] / nvox[a]) + 1.5);
-  return make_int3(r[0], r[1], r[2]);
+template <bool kFill>
+cudaError_t launch_voxels(const CellGeom& cell, const int* nvox, const double4* fw, const int* ftype, int nf,
+                          double lim2, int* counts, const int* off, int* atoms, unsigned short* atoms16, double4* xyzq,
+                          unsigned char* vtype, long long cap, cudaStream_t st) {
+  const int nv = nvox[0] * nvox[1] * nvox[2], warps = kVoxThreads / 32;
+  const bool ortho = cell.imcon == 1 || cell.imcon == 2;
+  VoxelCell f = {};
+  if (ortho) {
+    double h = 0.0;
+    for (int a = 0; a < 3; a++) {
+      const int i = cell.imcon == 1 ? 0 : a;
+      f.h[a] = (float)cell.h[4 * i];
+      f.r[a] = (float)cell.inv[i];
+      h = std::max(h, std::fabs(cell.h[4 * i]));
+    }
+    f.lim = (float)lim2;
+    f.scale = (float)(4.4e-6 * h);
+  }
+  const int per = warps * (ortho ? kVoxPerWarp<true> : kVoxPerWarp<false>);
+  const auto k = ortho ? fmc_voxel_kernel<true, kFill> : fmc_voxel_kernel<false, kFill>;
+  k<<<(nv + per - 1) / per, kVoxThreads, 0, st>>>(cell, f, nvox[0], nvox[1], nvox[2], fw, ftype, nf, lim2, counts, off,
+                                                  atoms, atoms16, xyzq, vtype, cap);
+  return cudaGetLastError();
 }
 }  // namespace
 
-bool voxel_prefilter_applies(const CellGeom& cell, const int* nvox) {
-  if (cell.imcon != 1 && cell.imcon != 2) return false;
-  for (int a = 0; a < 3; a++)
-    if (nvox[a] < 1 || nvox[a] > 1023 || !(cell.h[4 * a] > 0.0)) return false;
-  return true;
-}
-
-cudaError_t launch_voxel_codes(const CellGeom& cell, const int* nvox, const double4* fw, int nf, unsigned* code,
-                               cudaStream_t st) {
-  if (nf > 0)
-    fmc_voxel_code_kernel<<<(nf + kVoxThreads - 1) / kVoxThreads, kVoxThreads, 0, st>>>(cell, nvox[0], nvox[1],
-                                                                                       nvox[2], fw, nf, code);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_voxel_count(const CellGeom& cell, const int* nvox, const double4* fw, int nf, double lim2,
-                               const unsigned* code, int* counts, cudaStream_t st) {
-  int nv = nvox[0] * nvox[1] * nvox[2];
-  if (code && !voxel_prefilter_applies(cell, nvox)) code = nullptr;
-  const int3 r = code ? voxel_reach(cell, nvox, lim2) : make_int3(0, 0, 0);
-  fmc_voxel_count_kernel<<<nv, kVoxThreads, 0, st>>>(cell, nvox[0], nvox[1], nvox[2], fw, nf, lim2, code, r, counts);
-  return cudaGetLastError();
+                               int* counts, cudaStream_t st) {
+  if (nf < 1) return cudaMemsetAsync(counts, 0, sizeof(int) * nvox[0] * nvox[1] * nvox[2], st);
+  return launch_voxels<false>(cell, nvox, fw, nullptr, nf, lim2, counts, nullptr, nullptr, nullptr, nullptr, nullptr, 0, st);
 }
 
 cudaError_t launch_voxel_fill(const CellGeom& cell, const int* nvox, const double4* fw, const int* ftype, int nf,
-                              double lim2, const unsigned* code, const int* off, int* atoms, unsigned short* atoms16,
-                              double4* xyzq, unsigned char* vtype, long long cap, cudaStream_t st) {
-  int nv = nvox[0] * nvox[1] * nvox[2];
-  if (code && !voxel_prefilter_applies(cell, nvox)) code = nullptr;
-  const int3 r = code ? voxel_reach(cell, nvox, lim2) : make_int3(0, 0, 0);
-  fmc_voxel_fill_kernel<<<nv, kVoxThreads, 0, st>>>(cell, nvox[0], nvox[1], nvox[2], fw, ftype, nf, lim2, code, r,
-                                                    off, atoms, atoms16, xyzq, vtype, cap);
-  return cudaGetLastError();
+                              double lim2, const int* off, int* atoms, unsigned short* atoms16, double4* xyzq,
+                              unsigned char* vtype, long long cap, cudaStream_t st) {
+  return launch_voxels<true>(cell, nvox, fw, ftype, nf, lim2, nullptr, off, atoms, atoms16, xyzq, vtype, cap, st);
 }
 
 namespace {

@@ -126,18 +126,12 @@ cudaError_t launch_single_point_rs(const DevSystem& S, const GuestView& G, const
                                    cudaStream_t st);
 
 // Voxel lists: per voxel, the framework atoms within sqrt(lim2) of its centre by true minimum
-// image, in ascending atom order.  Orthorhombic cells (voxel_prefilter_applies) can pass
-// per-atom voxel codes (launch_voxel_codes, nf words) so that the FP64 test runs only for atoms
-// within reach; code = nullptr tests every atom.  Both give the same lists.
-bool voxel_prefilter_applies(const CellGeom& cell, const int* nvox);
-cudaError_t launch_voxel_codes(const CellGeom& cell, const int* nvox, const double4* fw, int nf, unsigned* code,
-                               cudaStream_t st);
+// image, in ascending atom order.
 cudaError_t launch_voxel_count(const CellGeom& cell, const int* nvox, const double4* fw, int nf, double lim2,
-                               const unsigned* code, int* counts, cudaStream_t st);
+                               int* counts, cudaStream_t st);
 cudaError_t launch_voxel_fill(const CellGeom& cell, const int* nvox, const double4* fw, const int* ftype, int nf,
-                              double lim2, const unsigned* code, const int* off, int* atoms, unsigned short* atoms16,
-                              double4* xyzq, unsigned char* vtype, long long cap,
-                              cudaStream_t st);  // entries >= cap not written
+                              double lim2, const int* off, int* atoms, unsigned short* atoms16, double4* xyzq,
+                              unsigned char* vtype, long long cap, cudaStream_t st);  // entries >= cap not written
 // The {erc, vvv} rows of DevSystem::pair_tab: rows * stride entries, row r holding vvv's row r
 // (row 0: no vdW table).
 cudaError_t launch_pack_tables(const double* erc, const double* vvv, int stride, int rows, double2* out,

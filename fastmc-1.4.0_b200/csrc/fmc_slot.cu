@@ -181,11 +181,9 @@ int build_slot(const HostSystem& h, int slot, const int seed[4], SlotMemory& mem
   unsigned char* d = nullptr;
   const int nv = h.nvox[0] * h.nvox[1] * h.nvox[2];
   if (vox_cap <= 0) vox_cap = slot_voxel_capacity(h);
-  const bool prefilter = voxel_prefilter_applies(h.cell, h.nvox) && h.nf > 0;
   v.K = h.K;
   for (int a = 0; a < 3; a++) v.kmax[a] = h.deck.kmax[a];
   int* counts = nullptr;
-  unsigned* code = nullptr;
   int* off = nullptr;
   double4* xyzq = nullptr;
   unsigned char* vt = nullptr;
@@ -195,8 +193,7 @@ int build_slot(const HostSystem& h, int slot, const int seed[4], SlotMemory& mem
   double* parts = nullptr;
   {
     // every buffer of the slot, set-up scratch included, from one pool allocation
-    const size_t arena = total + al(sizeof(int) * nv) + (prefilter ? al(sizeof(unsigned) * h.nf) : 0) +
-                         al(sizeof(int) * (nv + 1)) + al(sizeof(double4) * vox_cap) + al(vox_cap) +
+    const size_t arena = total + al(sizeof(int) * nv) + al(sizeof(int) * (nv + 1)) + al(sizeof(double4) * vox_cap) + al(vox_cap) +
                          al(sizeof(double2) * std::max(h.K, 1)) + al(sizeof(double2) * h.vvv.size()) +
                          al(sizeof(double) * std::max<size_t>(recip_scratch_doubles(v, h.nf), 1)) +
                          al(sizeof(double) * (recip_nparts(v) + 1)) + chain_state_bytes(h.deck, h, true) + 16 * 256;
@@ -218,14 +215,10 @@ int build_slot(const HostSystem& h, int slot, const int seed[4], SlotMemory& mem
   if ((e = mem.alloc((void**)&off, sizeof(int) * (nv + 1))) != cudaSuccess) goto fail;
   if ((e = mem.alloc((void**)&xyzq, sizeof(double4) * vox_cap)) != cudaSuccess) goto fail;
   if ((e = mem.alloc((void**)&vt, vox_cap)) != cudaSuccess) goto fail;
-  if (prefilter) {
-    if ((e = mem.alloc((void**)&code, sizeof(unsigned) * h.nf)) != cudaSuccess) goto fail;
-    e = launch_voxel_codes(h.cell, h.nvox, v.fw, h.nf, code, st);
-  }
-  if (e == cudaSuccess) e = launch_voxel_count(h.cell, h.nvox, v.fw, h.nf, h.vox_lim2, code, counts, st);
+  e = launch_voxel_count(h.cell, h.nvox, v.fw, h.nf, h.vox_lim2, counts, st);
   if (e == cudaSuccess) e = launch_exclusive_scan(counts, nv, off, st);
   if (e == cudaSuccess)
-    e = launch_voxel_fill(h.cell, h.nvox, v.fw, v.fw_type, h.nf, h.vox_lim2, code, off, nullptr, nullptr, xyzq, vt,
+    e = launch_voxel_fill(h.cell, h.nvox, v.fw, v.fw_type, h.nf, h.vox_lim2, off, nullptr, nullptr, xyzq, vt,
                           vox_cap, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(vox_total, off + nv, sizeof(int), cudaMemcpyDeviceToHost, st);
   if (e != cudaSuccess) goto fail;
