@@ -18,7 +18,8 @@ constexpr int kBatchMaxTypes = 16;  // unique atom types
 constexpr int kBatchMaxTab = kBatchMaxTypes * (kBatchMaxTypes + 1) / 2;
 // Tile shapes of the batched kernel the autotuner chooses among: threads per chain (CTA size),
 // k-vectors each thread takes per trip of the reciprocal loop (ewald.f:145-331) and neighbour
-// candidates per trip of the real-space loop (ewald.f:656-690, vdw_terms.f:455-495).  Tile 0
+// candidates per trip of the real-space loop (ewald.f:656-690, vdw_terms.f:455-495), of which a
+// warp takes 32 at a time and kChunksPerTrip more are always in flight.  Tile 0
 // is the default.  Within one thread-count the tiles give bit-identical results (each thread
 // sums its k-vectors and candidates in the same order); another thread count sums in another
 // order.  One chain per CTA throughout: two chains share an SM as two CTAs.

@@ -6,11 +6,12 @@
 //                     scratch, akk*(|S_new|^2-|S_old|^2) reduced per block.  Blocks [nbk, ...)
 //                     compute the real-space erfc Coulomb + tabulated vdW energy of one
 //                     trial site each (ewald2 + srfrce over the neighbour set that
-//                     guestlistgen would build).  The last block to finish combines the
-//                     block partials in a fixed order (deterministic) into {ewld1, ewld2, vdw}.
+//                     guestlistgen would build).  Each block puts its sums, stamped, into pinned
+//                     host memory; the host adds them in block order (deterministic).
 // fmc_commit_kernel : S(k) <- S_new and the guest-site array update of an accepted move.
 // fmc_recip_*       : full S(k) of a set of atoms (ewald1, ewald.f:368-630).
 // fmc_sp_kernel     : per-guest-site real-space energies for the single-point energy.
+// fmc_voxel_kernel  : the framework's per-voxel neighbour lists.
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
