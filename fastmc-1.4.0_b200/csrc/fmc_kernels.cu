@@ -764,7 +764,7 @@ __device__ __forceinline__ void voxel_centre(const CellGeom& c, int v, int n0, i
 // the longest period and s the largest |atom| + |centre| + h of an axis: rounding the coordinates, their
 // difference and n periods moves a separation by at most 3 * 2^-24 s and its square by h times that; where
 // it picks the other of two images, the square moves by at most 2^-21 h s.  Three axes: 2.2e-6 h s in all,
-// half of the margin.
+// half of the margin.  Atoms 2^16 periods out and further are left to double.
 // Bound by instructions issued (a test is some 20, and 3 for the atom's conversions) and, in the fill, by
 // stores of the two or so of 32 atoms that are in a list.  5,928 atoms and 28,656 lists: count 238 us, fill 560
 // us, against 517 and 1,112 with a block a voxel, a prefilter by voxel and four barriers every 128 atoms;
@@ -776,7 +776,7 @@ template <bool kOrtho>
 constexpr int kVoxPerWarp = kOrtho ? 2 : 1;
 
 struct VoxelCell {  // an orthorhombic cell's side of the float test, converted on the host: conversions are slow
-  float h[3], r[3], lim, scale;  // scale: 4.4e-6 h
+  float h[3], r[3], lim, scale, far;  // scale: 4.4e-6 h; far: 2^16 h, beyond which double decides alone
 };
 
 struct VoxelCentre {
@@ -793,7 +793,8 @@ __device__ __forceinline__ void voxel_flags(const CellGeom& c, const VoxelCell& 
   if (kOrtho) {
     constexpr float kRound = 12582912.0f;  // 1.5 * 2^23: adding it rounds to the nearest integer
     const float ax = (float)a.x, ay = (float)a.y, az = (float)a.z;
-    const float margin = f.scale * fmaxf(fabsf(ax), fmaxf(fabsf(ay), fabsf(az)));
+    const float out = fmaxf(fabsf(ax), fmaxf(fabsf(ay), fabsf(az)));
+    const float margin = out < f.far ? f.scale * out : __int_as_float(0x7f800000);
 #pragma unroll
     for (int u = 0; u < V; u++) {
       float dx = t[u].x - ax, dy = t[u].y - ay, dz = t[u].z - az;
@@ -911,6 +912,7 @@ cudaError_t launch_voxels(const CellGeom& cell, const int* nvox, const double4* 
     }
     f.lim = (float)lim2;
     f.scale = (float)(4.4e-6 * h);
+    f.far = (float)(65536.0 * h);
   }
   const int per = warps * (ortho ? kVoxPerWarp<true> : kVoxPerWarp<false>);
   const auto k = ortho ? fmc_voxel_kernel<true, kFill> : fmc_voxel_kernel<false, kFill>;
