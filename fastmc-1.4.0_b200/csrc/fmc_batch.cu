@@ -27,6 +27,7 @@ namespace {
 // The trial being evaluated: what the energy sums read, written while the move is set up.
 struct MoveSmem {
   int mtype, g, nold, nnew, ns, ex_lo, ex_hi;
+  int still;  // the trial leaves the molecule where it is (real_space_residue)
   double r[7], dis_delr, dis_rot;  // the trial's random numbers and step sizes (select_move)
   // trial sites (old ones first): position, charge factor q r4pie0 (negative for the old sites of a
   // displacement, whose energies are subtracted) and atom type, times types + 1 (a row of prow)
@@ -367,28 +368,21 @@ __device__ __forceinline__ long long global_ns() {
   return (long long)t;
 }
 
-// One warp: phase tables of the trial sites (ewald.f:95-137).  The first axis carries the site's
-// charge, negative for a site that leaves, so that the reciprocal loop only multiplies and adds.
+// One warp: phase tables of the trial sites (ewald.f:95-137).
 __device__ __forceinline__ void build_phases(const BatchSmem& B, double2* tab, int stride, int lane) {
   const MoveSmem& M = B.M;
   const DevSystem& S = B.Y.S;
-  const int nold = M.nold, nsite = nold + M.nnew, k1 = S.kmax[0], k2 = S.kmax[1];
-  const SpeciesConst& P = B.Y.sp[M.g];
+  const int nsite = M.nold + M.nnew, k1 = S.kmax[0], k2 = S.kmax[1];
 #pragma unroll 1
   for (int w = lane; w < nsite * 3; w += 32) {
     int st = w / 3, ax = w % 3;
     double f[3];
     frac_coords(S.cell, M.x[st], M.y[st], M.z[st], f);
     int off = st * stride + (ax == 0 ? 0 : (ax == 1 ? k1 + 1 : k1 + k2 + 2));
-    const double q = ax ? 1.0 : (st < nold ? -P.q[st] : P.q[st - nold]);
-    axis_phases(f[ax], S.kmax[ax], tab + off, q);
+    axis_phases(f[ax], S.kmax[ax], tab + off);
   }
 }
 
-// Warp 0: the serial part of a move's set-up (gcmc.f:753-847): species and move choice, step-size
-// adaptation, the counters it reads, and every random number of the trial in the reference's order
-// (utility_pack.f:2545-3000), left in r for the warp to build the trial sites from.  Every lane
-// takes the same branches and lane 0 writes.  `skip`: the last move's acceptance test took a draw.
 // Past the 32nd draw (a multi-jump that keeps drawing its first molecule): the state moves on.
 __device__ __noinline__ DrawWarp refill_draws(DrawWarp R, int lane) {
   Duni& d = batch_smem().C.rng;
@@ -422,6 +416,10 @@ __device__ __noinline__ void adapt_steps(int g) {
   }
 }
 
+// Warp 0: the serial part of a move's set-up (gcmc.f:753-847): species and move choice, step-size
+// adaptation, the counters it reads, and every random number of the trial in the reference's order
+// (utility_pack.f:2545-3000), left in r for the warp to build the trial sites from.  Every lane
+// takes the same branches and lane 0 writes.  `skip`: the last move's acceptance test took a draw.
 __device__ __noinline__ void select_move(int par, int skip, bool second, int lane) {
   BatchSmem& B = batch_smem();
   ChainDev& C = B.C;
@@ -591,6 +589,7 @@ __device__ __noinline__ void build_trial(int lane) {
     M.cq[lane] = (nnew ? -P.q[lane] : P.q[lane]) * kR4pie0;
     M.type[lane] = P.type[lane] * (S.ntypes + 1);
   }
+  bool still = false;
   if (nnew) {
     // one code path for every move type, so that it stays small: the site about the centre of
     // rotation (vx, vy, vz), the centre, the angle
@@ -635,6 +634,8 @@ __device__ __noinline__ void build_trial(int lane) {
       cm[1] = wy;
       cm[2] = wz;
       turn = M.dis_rot;
+      // draws are multiples of 2^-24, so an angle is now and then exactly zero
+      still = (M.dis_delr == 0.0 || (r[0] == 0.5 && r[1] == 0.5 && r[2] == 0.5)) && (ns == 1 || r[3] == 0.0 || turn == 0.0);
     }
     double q[4];
     axis_angle_quat(r[3] * turn, r[4], r[5], r[6], q);
@@ -677,42 +678,50 @@ __device__ __noinline__ void build_trial(int lane) {
   if (lane == 0) {
     M.nfw = fw;
     M.gchunks = gchunks;
+    M.still = still;
   }
 }
 
 // ------------------------------------------------------------------ energy sums of a trial
 // A thread's share of the reciprocal change (ewald.f:139-331): S_new(k) = S(k) + dS(k) to Sn, and akk
-// and |S_new|^2 - |S|^2 (ewald.f:311-319) returned.  A thread takes k-vectors tid, tid + NT, ... and adds their terms in that
-// order, KPT of them in flight.  Bound by the latency of its shared-memory reads and FP64 chain with
-// 1-4 k-vectors a thread, so the site loop is unrolled and the products go straight into the sums.
+// and |S_new|^2 - |S|^2 (ewald.f:311-319) returned.  A thread takes k-vectors tid, tid + NT, ... and adds
+// their terms in that order, KPT of them in flight.  Bound by the latency of its shared-memory reads and FP64
+// chain with 1-4 k-vectors a thread.
+//
+// The arithmetic is fixed, fma by fma: S(k) goes through every accepted move, and its last bits decide the
+// moves whose energy change is rounding alone (real_space_residue).  So the old and the new sites' terms are
+// summed apart, each q e^{ik.r} formed before it is added, and (S - old) + new taken in that order, in every
+// compiled tile.
 __device__ __forceinline__ double flip_sign(double v, int mask) {
   return __hiloint2double(__double2hiint(v) ^ mask, __double2loint(v));
 }
 
-// Sums over sites and k-vectors are written as fma: what the compiler contracts may differ between
-// the kernel's compiled tiles, which agree bit for bit.
-__device__ __forceinline__ double2 recip_term(int k, int nsite, int k1, int k2, int stride, const double2* tb,
-                                             const int* kp, const double* ak, const double2* Sk, double2* Sn) {
+__device__ __forceinline__ double2 recip_term(int k, const double* charge, int nold, int nsite, int k1, int k2,
+                                             int stride, const double2* tb, const int* kp, const double* ak,
+                                             const double2* Sk, double2* Sn) {
   int l, m, n;
   kunpack(kp[k], l, m, n);
   const int o2 = k1 + 1 + (m < 0 ? -m : m), o3 = k1 + k2 + 2 + (n < 0 ? -n : n);
   const int sm = m & 0x80000000, sn = n & 0x80000000;
-  double ax = 0.0, ay = 0.0;
+  double ax = 0.0, ay = 0.0, bx = 0.0, by = 0.0;  // the old sites' sum goes to b once it is complete
   const double2* t = tb;
+  const double* qp = charge;
 #pragma unroll 1
   for (int st = 0; st < nsite; st++, t += stride) {
     const double2 e1 = t[l], e2 = t[o2], e3 = t[o3];
-    const double y2 = flip_sign(e2.y, sm), y3 = flip_sign(e3.y, sn);
-    const double cx = fma(-e1.y, y2, e1.x * e2.x), cy = fma(e1.x, y2, e1.y * e2.x);
-    ax = fma(cx, e3.x, ax);
-    ay = fma(cy, e3.x, ay);
-    ax = fma(-cy, y3, ax);
-    ay = fma(cx, y3, ay);
+    const double q = *qp++, y2 = flip_sign(e2.y, sm), y3 = flip_sign(e3.y, sn);
+    const double px = fma(e1.x, e2.x, -(e1.y * y2)), py = fma(e1.y, e2.x, e1.x * y2);
+    ax = fma(q, fma(px, e3.x, -(py * y3)), ax);
+    ay = fma(q, fma(py, e3.x, px * y3), ay);
+    if (st == nold - 1) {
+      bx = ax;
+      by = ay;
+      ax = ay = 0.0;
+      qp = charge;
+    }
   }
-  const double2 so = Sk[k], sw = make_double2(so.x + ax, so.y + ay);
+  const double2 so = Sk[k], sw = make_double2((so.x - bx) + ax, (so.y - by) + ay);
   Sn[k] = sw;
-  // one order of roundings: uncharged molecules leave S(k) as it is, and what rounds off here decides
-  // their moves without an energy change (real_space_residue)
   return make_double2(ak[k], fma(-so.y, so.y, fma(-so.x, so.x, fma(sw.x, sw.x, sw.y * sw.y))));
 }
 
@@ -819,22 +828,26 @@ __device__ __forceinline__ void real_space(const BatchSmem& B, double& v1, doubl
   }
 }
 
-// The rotation of a single-site molecule changes no energy: what is left of E_new - E_old is the
-// rounding of two sums of the same pairs, yet its sign decides whether the acceptance test draws a
-// random number (gcmc.f:1330-1338).  So that seeded trajectories of uncharged molecules of that kind
-// stay what they are, these pairs keep one fixed arithmetic and order of addition: candidates tid, tid + NT, ... of the
-// old site's list and guests, then the new site's, correctly rounded roots, one table at a time.
+// A trial that leaves its molecule in place -- a single site's rotation, a rotation by a draw of exactly zero, a
+// translation with no step size -- changes no energy: what is left of E_new - E_old is the rounding of two sums of
+// the same pairs, yet its sign decides whether the acceptance test draws a random number (gcmc.f:1330-1338), and
+// so where a seeded chain goes from there.  These pairs keep one fixed arithmetic and order of addition:
+// candidates tid, tid + NT, ... of the old sites' lists, each followed by the guests, then the new sites', correctly
+// rounded roots, one table at a time.
 template <int NT>
 __device__ __noinline__ void real_space_residue(double* vout) {
   const BatchSmem& B = batch_smem();
   const MoveSmem& M = B.M;
   const DevSystem& S = B.Y.S;
-  const int gt = M.gpre[B.Y.nspecies], T0 = M.list[0].z + gt, T = T0 + M.list[1].z + gt;
-  const double chgea = B.Y.sp[M.g].q[0] * kR4pie0;
+  const int gt = M.gpre[B.Y.nspecies], ns = M.ns, nsite = 2 * ns;
   double v1 = 0.0, v2 = 0.0;
+  int s = 0, begin = 0;
 #pragma unroll 1
-  for (int t = threadIdx.x; t < T; t += NT) {
-    const int s = t >= T0, j = t - (s ? T0 : 0);
+  for (int t = threadIdx.x;; t += NT) {
+    while (s < nsite && t >= begin + M.list[s].z + gt) begin += M.list[s++].z + gt;
+    if (s >= nsite) break;
+    const int j = t - begin;
+    const double chgea = B.Y.sp[M.g].q[s < ns ? s : s - ns] * kR4pie0;
     double4 a;
     int type;
     const int4 d = M.list[s];
@@ -854,7 +867,8 @@ __device__ __noinline__ void real_space_residue(double* vout) {
     double ec = 0.0, ev = 0.0;
     double dx = M.x[s] - a.x, dy = M.y[s] - a.y, dz = M.z[s] - a.z;
     min_image(S.cell, dx, dy, dz);
-    const double rsq = fma(dz, dz, fma(dx, dx, dy * dy));
+    const bool xy = S.cell.imcon <= 3;
+    const double rsq = fma(dz, dz, xy ? fma(dx, dx, dy * dy) : fma(dy, dy, dx * dx));
     if (rsq < S.rcut2) {
       const double r = sqrt(rsq), chgprd = chgea * a.w;
       auto interp = [r](const double* tab, double rdr) {
@@ -868,7 +882,7 @@ __device__ __noinline__ void real_space_residue(double* vout) {
       if (fabs(chgprd) > 1e-10) ec = __dmul_rn(interp(S.erc, S.rdr_e), chgprd);
       if (off) ev = interp(S.vvv + off, S.rdr_v);
     }
-    if (s == 0) {
+    if (s < ns) {
       v1 -= ec;
       v2 -= ev;
     } else {
@@ -886,9 +900,12 @@ __device__ __noinline__ void sums_kind(int kmax_smem, int stride) {
   BatchSmem& B = batch_smem();
   const BatchArrays A = batch_arrays(kmax_smem);
   const DevSystem& S = B.Y.S;
-  const int tid = threadIdx.x, K = S.K, k1 = S.kmax[0], k2 = S.kmax[1], nsite = B.M.nold + B.M.nnew;
+  const int tid = threadIdx.x, K = S.K, k1 = S.kmax[0], k2 = S.kmax[1], nold = B.M.nold, nsite = nold + B.M.nnew;
+  const double* charge = B.Y.sp[B.M.g].q;
   double v0 = 0.0, v1 = 0.0, v2 = 0.0;
-  auto term = [&](int k) { return recip_term(k, nsite, k1, k2, stride, A.tab, A.kp, A.ak, A.Sk, A.Sn); };
+  auto term = [&](int k) {
+    return recip_term(k, charge, nold, nsite, k1, k2, stride, A.tab, A.kp, A.ak, A.Sk, A.Sn);
+  };
   int k = tid;
   if (KPT == 2)
 #pragma unroll 1
@@ -901,7 +918,7 @@ __device__ __noinline__ void sums_kind(int kmax_smem, int stride) {
     const double2 a = term(k);
     v0 = fma(a.x, a.y, v0);
   }
-  if (B.M.ns == 1 && B.M.mtype == kRotate) {
+  if (B.M.still) {
     double v[2];
     real_space_residue<NT>(v);
     v1 = v[0];

@@ -77,12 +77,12 @@ __device__ __forceinline__ double2 cmulc(double2 a, double2 b) {  // a * conj(b)
   return make_double2(a.x * b.x + a.y * b.y, a.y * b.x - b.y * a.x);
 }
 
-// q e^{i 2 pi j s} for j = 0..kmax by the recurrence of ewald.f:118-137 into tab[0..kmax].
-__device__ __forceinline__ void axis_phases(double s, int kmax, double2* tab, double q = 1.0) {
+// e^{i 2 pi j s} for j = 0..kmax by the recurrence of ewald.f:118-137 into tab[0..kmax].
+__device__ __forceinline__ void axis_phases(double s, int kmax, double2* tab) {
   double sn, cs;
   sincos(2.0 * kPi * s, &sn, &cs);
-  tab[0] = make_double2(q, 0.0);
-  double2 p = make_double2(q * cs, q * sn);
+  tab[0] = make_double2(1.0, 0.0);
+  double2 p = make_double2(cs, sn);
   if (kmax >= 1) tab[1] = p;
 #pragma unroll 1
   for (int j = 2; j <= kmax; j++) {
