@@ -234,8 +234,9 @@ struct PendingCommit {
 // Thread-partial real-space energy of one site against the framework (voxel list) and the
 // guest sites outside [ex_lo, ex_hi).  Threads stride by `nthr` starting at `tid`.
 //
-// Single-site molecules only (pass_block): their moves without an energy change are decided by what
-// these sums round off, so they keep this arithmetic and order.
+// For single-site molecules and for trials that leave a molecule in place (a rotation by a draw of exactly zero, a
+// translation with no step size): what these sums round off decides such a move's acceptance test, and so
+// where a seeded chain goes from there, so they keep this arithmetic and order.
 __device__ __forceinline__ void site_partial(const DevSystem& S, const GuestView& G, const PendingCommit& P, double px,
                                              double py, double pz, double q, int ty, int vb, int vl, int ex_lo,
                                              int ex_hi, int tid, int nthr, double& ec_fw, double& ev_fw, double& ec_g, double& ev_g) {

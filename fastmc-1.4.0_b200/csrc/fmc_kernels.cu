@@ -113,31 +113,29 @@ __device__ __forceinline__ bool pass_block(const DevSystem& S, const GuestView& 
       int l, m, n;
       kunpack(kp, l, m, n);
       int am = m < 0 ? -m : m, an = n < 0 ? -n : n;
-      double2 aold = make_double2(0.0, 0.0), anew = make_double2(0.0, 0.0);
+      // the arithmetic is fixed, fma by fma, and the old and new sites' terms are summed apart: S(k) goes through
+      // every accepted move, and its last bits decide the moves whose energy change is rounding alone (site_partial)
+      const int mneg = m & 0x80000000, nneg = n & 0x80000000;
+      double ax = 0.0, ay = 0.0, bx = 0.0, by = 0.0;  // the old sites' sum goes to b once it is complete
 #pragma unroll 3
       for (int s = 0; s < nsite; s++) {
         const double2* t = sm_tab + s * stride;
-        double2 e1 = t[l], e2 = t[k1 + 1 + am], e3 = t[k1 + k2 + 2 + an];
-        double2 c = m >= 0 ? cmul(e1, e2) : cmulc(e1, e2);
-        c = n >= 0 ? cmul(c, e3) : cmulc(c, e3);
-        double q = A.q[s];
-        if (s < A.nold) {
-          aold.x += q * c.x;
-          aold.y += q * c.y;
-        } else {
-          anew.x += q * c.x;
-          anew.y += q * c.y;
+        const double2 e1 = t[l], e2 = t[k1 + 1 + am], e3 = t[k1 + k2 + 2 + an];
+        const double q = A.q[s], y2 = __hiloint2double(__double2hiint(e2.y) ^ mneg, __double2loint(e2.y)),
+                     y3 = __hiloint2double(__double2hiint(e3.y) ^ nneg, __double2loint(e3.y));
+        const double px = fma(e1.x, e2.x, -(e1.y * y2)), py = fma(e1.y, e2.x, e1.x * y2);
+        const double cp = fma(px, y3, py * e3.x), cm = fma(py, e3.x, px * y3);
+        ax = fma(q, fma(px, e3.x, -(py * y3)), ax);
+        ay = fma(q, nneg ? cm : cp, ay);
+        if (s == A.nold - 1) {
+          bx = ax;
+          by = ay;
+          ax = ay = 0.0;
         }
       }
-      double2 sn;
-      if (A.move == kInsert)
-        sn = make_double2(anew.x + so.x, anew.y + so.y);
-      else if (A.move == kDelete)
-        sn = make_double2(so.x - aold.x, so.y - aold.y);
-      else
-        sn = make_double2((so.x - aold.x) + anew.x, (so.y - aold.y) + anew.y);
+      const double2 sn = make_double2((so.x - bx) + ax, (so.y - by) + ay);
       sk_new[k] = sn;
-      v[0] = ak * (sn.x * sn.x + sn.y * sn.y - so.x * so.x - so.y * so.y);
+      v[0] = ak * fma(-so.y, so.y, fma(-so.x, so.x, fma(sn.x, sn.x, sn.y * sn.y)));
     }
     block_sum<1>(v, sm.red);
     if (tid == 0) publish(W.recip_slot(blk), v[0], pass_stamp(A.seq, v[0], 0.0));
@@ -146,7 +144,7 @@ __device__ __forceinline__ bool pass_block(const DevSystem& S, const GuestView& 
     const int s = blk - nbk;
     double v[2] = {0.0, 0.0};
     double ec_fw = 0.0, ev_fw = 0.0, ec_g = 0.0, ev_g = 0.0;
-    if (A.single) {
+    if (A.fixed) {
       site_partial(S, G, A.pc, A.x[s], A.y[s], A.z[s], A.q[s], A.type[s], A.vb[s], A.vl[s], A.ex_lo, A.ex_hi, tid,
                    blockDim.x, ec_fw, ev_fw, ec_g, ev_g);
     } else {

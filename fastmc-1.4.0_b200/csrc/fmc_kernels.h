@@ -21,7 +21,7 @@ struct PassArgsT {
   int do_real;        // 1: one real-space block per site
   int nold, nnew;
   int ex_lo, ex_hi;   // guest-site range of the moving molecule (excluded from real space)
-  int single, pad;    // a single-site molecule: real space in its fixed order (site_partial)
+  int fixed, pad;     // real space in its fixed order (site_partial)
   double engsic;      // self-interaction term of the species (ewald.f:87-93)
   double seq;         // the pass's number, which stamps its results (pass_stamp)
   double x[N], y[N], z[N], q[N];

@@ -116,7 +116,7 @@ def golden():
 
 
 @pytest.mark.parametrize("name", CASES)
-@pytest.mark.parametrize("path", ["batched"])
+@pytest.mark.parametrize("path", ["batched", "plain"])
 def test_still_moves_keep_their_bits(fmc, tmp_path, golden, name, path):
     from fastmc_b200 import synth
 
