@@ -189,6 +189,10 @@ __device__ __forceinline__ void pair_table(const DevSystem& S, double rs, double
   }
 }
 
+// The voxel of n that t falls into; t below 1, or no number, is voxel 0 (converting it to an int first would
+// give the host any value).
+FMC_HD int voxel_index(double t, int n) { return t >= 1.0 ? (t < (double)n ? (int)t : n - 1) : 0; }
+
 // Voxel of a position (wrapped into the cell; a slab's z clamped to its layers, whose lowest and
 // highest hold no atom).
 FMC_HD int voxel_of(const DevSystem& S, double x, double y, double z) {
@@ -197,21 +201,13 @@ FMC_HD int voxel_of(const DevSystem& S, double x, double y, double z) {
     const CellGeom& c = S.cell;
     s[0] = c.slab[0] * x + c.slab[2] * y;
     s[1] = c.slab[1] * x + c.slab[3] * y;
-    s[2] = 0.0;
-    double t = (z - c.zlo) * c.rdz;
-    int k = t < 0.0 ? 0 : (t >= (double)S.nvox[2] ? S.nvox[2] - 1 : (int)t);
-    int v0 = (int)((s[0] - floor(s[0])) * S.nvox[0]), v1 = (int)((s[1] - floor(s[1])) * S.nvox[1]);
-    v0 = v0 < 0 ? 0 : (v0 >= S.nvox[0] ? S.nvox[0] - 1 : v0);
-    v1 = v1 < 0 ? 0 : (v1 >= S.nvox[1] ? S.nvox[1] - 1 : v1);
-    return (v0 * S.nvox[1] + v1) * S.nvox[2] + k;
+    const int v0 = voxel_index((s[0] - floor(s[0])) * S.nvox[0], S.nvox[0]);
+    const int v1 = voxel_index((s[1] - floor(s[1])) * S.nvox[1], S.nvox[1]);
+    return (v0 * S.nvox[1] + v1) * S.nvox[2] + voxel_index((z - c.zlo) * c.rdz, S.nvox[2]);
   }
   frac_coords(S.cell, x, y, z, s);
   int v[3];
-  for (int a = 0; a < 3; a++) {
-    double f = s[a] - floor(s[a]);
-    int i = (int)(f * S.nvox[a]);
-    v[a] = i < 0 ? 0 : (i >= S.nvox[a] ? S.nvox[a] - 1 : i);
-  }
+  for (int a = 0; a < 3; a++) v[a] = voxel_index((s[a] - floor(s[a])) * S.nvox[a], S.nvox[a]);
   return (v[0] * S.nvox[1] + v[1]) * S.nvox[2] + v[2];
 }
 
