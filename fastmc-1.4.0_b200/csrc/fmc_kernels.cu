@@ -603,7 +603,11 @@ cudaError_t launch_recip_full(const DevSystem& S, const AtomSegs& atoms, double2
   // octets once their blocks give every SM one: below that the launch lasts as long as one thread's
   // atoms, eight times shorter with one k-vector a thread
   const int bx = (S.noct + kOctetThreads - 1) / kOctetThreads;
-  if (bx * nchunk >= 148)
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  if ((long long)bx * nchunk >= sms)
     fmc_recip_octet_kernel<<<dim3(bx, nchunk), kOctetThreads, smem, st>>>(S, atoms, natoms, chunk, partial);
   else
     fmc_recip_single_kernel<<<dim3((S.K + kSingleThreads - 1) / kSingleThreads, nchunk), kSingleThreads, smem, st>>>(
