@@ -625,17 +625,6 @@ void Chain::place_sites(PassArgs& A) const {
   }
 }
 
-// The words of one block's slot, once their stamp is that of pass seq.
-static bool slot_arrived(const double* p, double seq, int n, double* out) {
-  const volatile double* v = p;
-  const double stamp = v[n];
-  double e[2] = {v[0], n > 1 ? v[1] : 0.0};
-  const double want = pass_stamp(seq, e[0], e[1]);
-  if (std::memcmp(&stamp, &want, sizeof(stamp))) return false;
-  std::copy(e, e + n, out);
-  return true;
-}
-
 bool Chain::collect(const PassArgs& A, const volatile int* ended, double out[3]) const {
   // block by block, in the order in which they are added; the wait for all of them is bounded (well over
   // a second)

@@ -5,6 +5,7 @@
 #pragma once
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 
 #if defined(__CUDACC__)
 #define FMC_HD __host__ __device__ __forceinline__
@@ -83,10 +84,14 @@ FMC_HD double duni_next(Duni& d) {
   return (double)uni;
 }
 
-// The stamp beside a block's energies a, b in pinned memory: the pass's number folded with their bits, so
+// The stamp beside a block's energies a, b in pinned memory: a hash of the pass's number and their bits, so
 // that a reader knows the words belong to pass `seq` in whatever order they arrived.  (Compared as
-// words: a double of any bits.)
+// words: a double of any bits.)  A number is a double of few bits, all at its top, and energies may be as short, so
+// each word is multiplied and its upper half folded down before the next one comes in: merely xored
+// together, the old stamp matched one new energy beside an old one (passes 1 and 2, -1.25 then
+// -0.01239013671875).  Given the rest, another number, a or b gives another stamp.
 FMC_HD double pass_stamp(double seq, double a, double b) {
+  constexpr unsigned long long kOdd = 0x9E3779B97F4A7C15ULL;  // 2^64 over the golden ratio
   union {
     double d;
     unsigned long long u;
@@ -94,9 +99,22 @@ FMC_HD double pass_stamp(double seq, double a, double b) {
   s.d = seq;
   x.d = a;
   y.d = b;
-  s.u *= 0x9E3779B97F4A7C15ULL;  // spreads the few bits in which two passes' numbers differ
-  s.u ^= (x.u << 7 | x.u >> 57) ^ (y.u << 23 | y.u >> 41);
+  s.u *= kOdd;
+  s.u = (s.u ^ s.u >> 32) * kOdd;
+  s.u = ((s.u ^ s.u >> 32) ^ x.u) * kOdd;
+  s.u = ((s.u ^ s.u >> 32) ^ y.u) * kOdd;
   return s.d;
+}
+
+// Takes the n (1 or 2) energies of a block's slot {energies, stamp} if their stamp is that of pass seq.
+inline bool slot_arrived(const double* p, double seq, int n, double* out) {
+  const volatile double* v = p;
+  const double stamp = v[n];
+  const double e[2] = {v[0], n > 1 ? v[1] : 0.0};
+  const double want = pass_stamp(seq, e[0], e[1]);
+  if (std::memcmp(&stamp, &want, sizeof(stamp))) return false;
+  for (int i = 0; i < n; i++) out[i] = e[i];
+  return true;
 }
 
 // ------------------------------------------------------------------ cell geometry
