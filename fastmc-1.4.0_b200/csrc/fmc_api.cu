@@ -234,7 +234,6 @@ int fmc_guest_realspace(fmc_chain* c, int iguest, int natms, const double* xyz, 
     A.q[i] = G.charge[i];
     A.type[i] = (unsigned char)G.type[i];
   }
-  A.fixed = natms == 1;
   A.seq = C.pass_seq += 1.0;
   C.place_sites(A);
   if (int rc0 = C.stop_server()) return fail(rc0, "the resident pass kernel did not end");

@@ -656,7 +656,7 @@ bool Chain::collect(const PassArgs& A, const volatile int* ended, double out[3])
   return true;
 }
 
-int Chain::pass(int move, int g, int mol, const double* old_xyz, const double* new_xyz, double out[3], bool still) {
+int Chain::pass(int move, int g, int mol, const double* old_xyz, const double* new_xyz, double out[3]) {
   PassArgs A;
   std::memset(&A, 0, sizeof(A));
   const GuestSpecies& G = sys.deck.guests[g];
@@ -672,7 +672,6 @@ int Chain::pass(int move, int g, int mol, const double* old_xyz, const double* n
     A.ex_hi = A.ex_lo + s.nsite;
   }
   A.engsic = sys.engsic[g];
-  A.fixed = s.nsite == 1 || still;
   int w = 0;
   for (int i = 0; i < A.nold; i++, w++) {
     A.x[w] = old_xyz[3 * i];
@@ -1108,10 +1107,7 @@ int Chain::step(MoveRecord* rec) {
       newx[3 * i + 1] = y[i];
       newx[3 * i + 2] = z[i];
     }
-    // draws are multiples of 2^-24, so an angle is now and then exactly zero
-    const bool still = (dis_delr == 0.0 || (r[0] == 0.5 && r[1] == 0.5 && r[2] == 0.5)) &&
-                       (natms == 1 || r[3] == 0.0 || dis_rot == 0.0);
-    if ((rc = pass(kDisplace, g, mol, oldx, newx, e, still))) return rc;
+    if ((rc = pass(kDisplace, g, mol, oldx, newx, e))) return rc;
     estep = (e[0] + e[1] + e[2]) / sys.engunit;
     if (estep < 0.0) {
       accepted = true;

@@ -103,9 +103,8 @@ class Chain {
   // open from a system already built on the host by prepare_system (the device part only)
   int open_prepared(HostSystem&& prepared, const int seed[4], int device, std::string& err);
   GuestView guest_view() const;
-  // Energies of one trial pass.  old_xyz/new_xyz are interleaved xyz of the molecule's sites.  still: the trial
-  // leaves the molecule in place, so that its energies keep one fixed order of rounding (site_partial).
-  int pass(int move, int g, int mol, const double* old_xyz, const double* new_xyz, double out[3], bool still = false);
+  // Energies of one trial pass.  old_xyz/new_xyz are interleaved xyz of the molecule's sites.
+  int pass(int move, int g, int mol, const double* old_xyz, const double* new_xyz, double out[3]);
   // An accepted move: S(k) <- S_new by exchanging the two buffers, and the guest-site update
   // left pending for the next pass to read through and write (no launch of its own); a second
   // update before the next pass, or one of more than kMaxPendSites sites, is written at once.

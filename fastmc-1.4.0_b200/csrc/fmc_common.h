@@ -604,6 +604,19 @@ FMC_HD double sqrt_refine(double x, double y) {
   return fma(fma(-g, g, x), h, g);
 }
 
+// The same with 1/(2 sqrt(x)) taken to full precision beside the first correction and a second one, of an ulp's
+// residual at most: rounded as sqrt(x) is.
+FMC_HD double sqrt_rounded(double x, double y) {
+  double g = x * y, h = 0.5 * y;
+  double r = fma(-h, g, 0.5);
+  g = fma(g, r, g);
+  h = fma(h, r, h);
+  r = fma(-h, g, 0.5);
+  g = fma(fma(-g, g, x), h, g);
+  h = fma(h, r, h);
+  return fma(fma(-g, g, x), h, g);
+}
+
 // 3-point interpolation of a tabulated function on r_l = l*dr (ewald.f:670-684,
 // vdw_terms.f:476-489).  tab[0] is defined as tab[1].
 FMC_HD double interp3(const double* tab, double rrr, double rdr) {

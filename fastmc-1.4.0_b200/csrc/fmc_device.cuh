@@ -91,13 +91,21 @@ __device__ __forceinline__ void axis_phases(double s, int kmax, double2* tab) {
   }
 }
 
-// sqrt(x) for x >= 0 without a branch: the hardware's estimate of 1/sqrt(x), refined.  The added
-// 1e-300 leaves every normal x as it is and keeps x = 0 finite.
-__device__ __forceinline__ double sqrt_approx(double x) {
+// sqrt(x) for x >= 0 without a branch, within an ulp or rounded correctly: the hardware's estimate of
+// 1/sqrt(x), refined.  The added 1e-300 leaves every x above 1e-284 as it is and keeps x = 0 finite.
+__device__ __forceinline__ double rsqrt_estimate(double& x) {
   double y;
   x += 1e-300;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+__device__ __forceinline__ double sqrt_approx(double x) {
+  const double y = rsqrt_estimate(x);
   return sqrt_refine(x, y);
+}
+__device__ __forceinline__ double sqrt_exact(double x) {
+  const double y = rsqrt_estimate(x);
+  return sqrt_rounded(x, y);
 }
 
 // Fractional coordinates s = rcell . r as in ewald.f:106-108.
@@ -106,22 +114,6 @@ FMC_HD void frac_coords(const CellGeom& c, double x, double y, double z, double*
   s[0] = r[0] * x + r[3] * y + r[6] * z;
   s[1] = r[1] * x + r[4] * y + r[7] * z;
   s[2] = r[2] * x + r[5] * y + r[8] * z;
-}
-
-// Pair energy of one site with charge factor chgea = q_i*r4pie0 and table row lookup base.
-// kImcon < 0: the boundary condition is read from the cell.
-template <int kImcon = -1>
-__device__ __forceinline__ void pair_energy(const DevSystem& S, double dx, double dy, double dz, double chgea,
-                                            double qj, int row, double& ec, double& ev) {
-  if (kImcon < 0) min_image(S.cell, dx, dy, dz);
-  else min_image_t<kImcon>(S.cell, dx, dy, dz);
-  double rsq = dx * dx + dy * dy + dz * dz;
-  if (rsq < S.rcut2) {
-    double r = sqrt(rsq);
-    double chgprd = chgea * qj;
-    if (fabs(chgprd) > 1e-10) ec += interp3(S.erc, r, S.rdr_e) * chgprd;
-    if (row >= 0) ev += interp3(S.vvv + (size_t)row * S.tab_stride, r, S.rdr_v);
-  }
 }
 
 // ------------------------------------------------------------------ pairs without branches
@@ -142,9 +134,9 @@ __device__ __forceinline__ double nint_rest(double x) {
   return fabs(f) == 0.5 ? copysign(0.5, -x) : f;
 }
 
-// Squared distance of the reference's image of a separation (images, utility_pack.f:1138-1349).
+// The reference's image of a separation (images, utility_pack.f:1138-1349).
 template <int KIND>
-__device__ __forceinline__ double image_dist2(const CellGeom& c, double dx, double dy, double dz) {
+__device__ __forceinline__ void image(const CellGeom& c, double& dx, double& dy, double& dz) {
   if (KIND == kPairOrtho) {
     // nint by the rounding of an addition: a tie picks either image, at the same distance; imcon 1
     // takes the first edge for every axis
@@ -163,6 +155,11 @@ __device__ __forceinline__ double image_dist2(const CellGeom& c, double dx, doub
   } else {
     min_image(c, dx, dy, dz);
   }
+}
+
+template <int KIND>
+__device__ __forceinline__ double image_dist2(const CellGeom& c, double dx, double dy, double dz) {
+  image<KIND>(c, dx, dy, dz);
   return fma(dx, dx, fma(dy, dy, dz * dz));
 }
 
@@ -227,46 +224,6 @@ struct PendingCommit {
   int type[kMaxPendSites];
 };
 
-// Thread-partial real-space energy of one site against the framework (voxel list) and the
-// guest sites outside [ex_lo, ex_hi).  Threads stride by `nthr` starting at `tid`.
-//
-// For single-site molecules and for trials that leave a molecule in place (a rotation by a draw of exactly zero, a
-// translation with no step size): what these sums round off decides such a move's acceptance test, and so
-// where a seeded chain goes from there, so they keep this arithmetic and order.
-__device__ __forceinline__ void site_partial(const DevSystem& S, const GuestView& G, const PendingCommit& P, double px,
-                                             double py, double pz, double q, int ty, int vb, int vl, int ex_lo,
-                                             int ex_hi, int tid, int nthr, double& ec_fw, double& ev_fw, double& ec_g, double& ev_g) {
-  const double chgea = q * kR4pie0;
-  const int* prow = S.pair_row + ty * (S.ntypes + 1);
-  for (int sg = 0; sg < G.nseg; sg++) {
-    int lo = G.seg_off[sg], hi = lo + G.seg_len[sg];
-    for (int j = lo + tid; j < hi; j += nthr) {
-      if (j >= ex_lo && j < ex_hi) continue;
-      double4 a;
-      int t;
-      if (sg != P.seg || j < P.lo) {
-        a = G.site[j];
-        t = G.type[j];
-      } else if (P.op == kDelete) {  // the sites after the removed molecule, one molecule on
-        a = G.site[j + P.ns];
-        t = G.type[j + P.ns];
-      } else if (j < P.lo + P.ns) {  // the inserted or displaced molecule
-        a = P.site[j - P.lo];
-        t = P.type[j - P.lo];
-      } else {
-        a = G.site[j];
-        t = G.type[j];
-      }
-      pair_energy(S, px - a.x, py - a.y, pz - a.z, chgea, a.w, prow[t], ec_g, ev_g);
-    }
-  }
-  const int b = vb, e = vb + vl;
-  for (int i = b + tid; i < e; i += nthr) {
-    double4 a = S.vox_xyzq[i];
-    pair_energy(S, px - a.x, py - a.y, pz - a.z, chgea, a.w, prow[S.vox_type[i]], ec_fw, ev_fw);
-  }
-}
-
 // The guest site j of segment sg as if the pending update were written.
 __device__ __forceinline__ void guest_site(const GuestView& G, const PendingCommit& P, int sg, int j, double4& a,
                                            int& t) {
@@ -281,6 +238,46 @@ __device__ __forceinline__ void guest_site(const GuestView& G, const PendingComm
   }
   a = G.site[j];
   t = G.type[j];
+}
+
+// The plain path's pairs keep one arithmetic, every bit of it: what a site's sum rounds off decides a move that leaves
+// its molecule in place (an angle drawn as exactly zero, any rotation of a single site), and so where a seeded
+// host loop goes from there, whether it runs in the library or calls the drop-in routines.  So the root is rounded
+// correctly and the roundings are written out; the images' products are fused as the compiler does.  A plain move
+// takes as long as with image_dist2 and pair_table (10.1 us, 424 atoms).
+template <int KIND>
+__device__ __forceinline__ double plain_dist2(const CellGeom& c, double dx, double dy, double dz) {
+  image<KIND>(c, dx, dy, dz);
+  return fma(dz, dz, fma(dy, dy, __dmul_rn(dx, dx)));
+}
+
+__device__ __forceinline__ double plain_interp(double v0, double v1, double v2, double p) {
+  const double t1 = fma(v1 - v0, p, v0), t2 = fma(v2 - v1, p - 1.0, v1);
+  return fma(__dmul_rn(t2 - t1, p), 0.5, t1);
+}
+
+// Adds a pair's table energies: ec += cq erc(r), ev += vvv(r), with rs and off as in pair_table.
+template <int KIND>
+__device__ __forceinline__ void plain_table(const DevSystem& S, double rs, double cq, int off, double& ec, double& ev) {
+  const double r = sqrt_exact(rs), x = __dmul_rn(r, S.rdr_e);
+  const double f = (x - 0.5) + kMagic;  // floor(x) but for integers
+  const int l = __double2loint(f);
+  const double p = x - (f - kMagic);
+  if (KIND != kPairGeneral) {
+    const double2* tb = S.pair_tab + (off + l);
+    const double2 a0 = tb[0], a1 = tb[1], a2 = tb[2];
+    ec = fma(plain_interp(a0.x, a1.x, a2.x, p), cq, ec);
+    ev = ev + plain_interp(a0.y, a1.y, a2.y, p);
+  } else {
+    const double* te = S.erc + l;
+    ec = fma(plain_interp(te[0], te[1], te[2], p), cq, ec);
+    if (off) {
+      const double xv = __dmul_rn(r, S.rdr_v);
+      const int lv = (int)xv;
+      const double* tv = S.vvv + (off + lv);
+      ev = ev + plain_interp(tv[0], tv[1], tv[2], xv - (double)lv);
+    }
+  }
 }
 
 // A thread's share of the pairs of one site with n candidates: two candidates in flight, distances
@@ -310,7 +307,7 @@ __device__ __forceinline__ void pair_sum(const DevSystem& S, const int* prow, do
     int off[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      const double rsq = image_dist2<KIND>(S.cell, px - a[u].x, py - a[u].y, pz - a[u].z);
+      const double rsq = plain_dist2<KIND>(S.cell, px - a[u].x, py - a[u].y, pz - a[u].z);
       const bool in = t[u] >= 0 && rsq < S.rcut2;
       const double qq = chgea * a[u].w;
       rs[u] = in ? rsq : S.rcut2;
@@ -318,7 +315,7 @@ __device__ __forceinline__ void pair_sum(const DevSystem& S, const int* prow, do
       off[u] = in ? prow[t[u]] : 0;
     }
 #pragma unroll
-    for (int u = 0; u < U; u++) pair_table<KIND>(S, rs[u], cq[u], off[u], 1.0, ec, ev);
+    for (int u = 0; u < U; u++) plain_table<KIND>(S, rs[u], cq[u], off[u], ec, ev);
     base += U * nthr;
   } while (base < n);
 }

@@ -114,7 +114,7 @@ __device__ __forceinline__ bool pass_block(const DevSystem& S, const GuestView& 
       kunpack(kp, l, m, n);
       int am = m < 0 ? -m : m, an = n < 0 ? -n : n;
       // the arithmetic is fixed, fma by fma, and the old and new sites' terms are summed apart: S(k) goes through
-      // every accepted move, and its last bits decide the moves whose energy change is rounding alone (site_partial)
+      // every accepted move, and its last bits decide the moves whose energy change is rounding alone (plain_dist2)
       const int mneg = m & 0x80000000, nneg = n & 0x80000000;
       double ax = 0.0, ay = 0.0, bx = 0.0, by = 0.0;  // the old sites' sum goes to b once it is complete
 #pragma unroll 3
@@ -144,24 +144,19 @@ __device__ __forceinline__ bool pass_block(const DevSystem& S, const GuestView& 
     const int s = blk - nbk;
     double v[2] = {0.0, 0.0};
     double ec_fw = 0.0, ev_fw = 0.0, ec_g = 0.0, ev_g = 0.0;
-    if (A.fixed) {
-      site_partial(S, G, A.pc, A.x[s], A.y[s], A.z[s], A.q[s], A.type[s], A.vb[s], A.vl[s], A.ex_lo, A.ex_hi, tid,
-                   blockDim.x, ec_fw, ev_fw, ec_g, ev_g);
-    } else {
-      const int row = tid <= S.ntypes ? max(S.pair_row[A.type[s] * (S.ntypes + 1) + tid], 0) * S.tab_stride : 0;
-      auto rows = [&]() {
-        if (tid <= S.ntypes) sm.prow[tid] = row;
-        __syncthreads();
-      };
-      const int kind = pair_kind(S);
-      auto pairs = [&](auto k) {
-        site_pairs<decltype(k)::value>(S, G, A.pc, sm.prow, A.x[s], A.y[s], A.z[s], A.q[s], A.vb[s], A.vl[s], A.ex_lo,
-                                       A.ex_hi, tid, blockDim.x, rows, ec_fw, ev_fw, ec_g, ev_g);
-      };
-      if (kind == kPairOrtho) pairs(std::integral_constant<int, kPairOrtho>());
-      else if (kind == kPairTriclinic) pairs(std::integral_constant<int, kPairTriclinic>());
-      else pairs(std::integral_constant<int, kPairGeneral>());
-    }
+    const int row = tid <= S.ntypes ? max(S.pair_row[A.type[s] * (S.ntypes + 1) + tid], 0) * S.tab_stride : 0;
+    auto rows = [&]() {
+      if (tid <= S.ntypes) sm.prow[tid] = row;
+      __syncthreads();
+    };
+    const int kind = pair_kind(S);
+    auto pairs = [&](auto k) {
+      site_pairs<decltype(k)::value>(S, G, A.pc, sm.prow, A.x[s], A.y[s], A.z[s], A.q[s], A.vb[s], A.vl[s], A.ex_lo,
+                                     A.ex_hi, tid, blockDim.x, rows, ec_fw, ev_fw, ec_g, ev_g);
+    };
+    if (kind == kPairOrtho) pairs(std::integral_constant<int, kPairOrtho>());
+    else if (kind == kPairTriclinic) pairs(std::integral_constant<int, kPairTriclinic>());
+    else pairs(std::integral_constant<int, kPairGeneral>());
     v[0] = ec_g + ec_fw;
     v[1] = ev_g + ev_fw;
     block_sum<2>(v, sm.red);

