@@ -420,8 +420,9 @@ def run_batched(args, dist):
         per_launch += args.moves * (inf["K"] * 40 + 4.5 * nrc * 36)
     avg_launch_s = t_dev / args.steps
     achieved = per_launch / avg_launch_s / 1e9
-    # ncu DRAM bytes per chain-move (captured on a 200-move launch), scaled to this launch
-    tpm = profiled_traffic("batch_kernel_batched", "traffic_bytes_per_chain_move")
+    # ncu DRAM bytes per chain-move at this voxel edge (captured on a 2,000-move launch of 32 of the chains),
+    # scaled to this launch; none where this edge has not been captured
+    tpm = profiled_traffic("batch_kernel_batched", f"traffic_bytes_per_chain_move at {edge:g} A")
     traffic = tpm * n * args.moves if tpm else None
     peak, peak_kind = peaks()
     from fastmc_b200._lib import lib as _l

@@ -10,8 +10,8 @@
 //
 // A chain's move is a serial chain of latencies; what one costs, in SM cycles (16 chains, one an SM,
 // K = 131, 510 atoms / 256 chains of 16 frameworks, two chains on most SMs): before the set-up and the
-// bookkeeping were split over warps 24.2k / 30.8k (set-up 7.0k / 8.3k, sums 12.6k / 17.6k, acceptance,
-// bookkeeping and commit 4.6k / 4.9k), now 14.5k / 20.6k.  Code that runs once a move comes through the
+// bookkeeping were split over warps 23.8k / 30.0k (set-up 7.0k / 8.3k, sums 12.5k / 17.0k, acceptance,
+// bookkeeping and commit 4.6k / 4.9k), now 14.8k / 19.2k.  Code that runs once a move comes through the
 // instruction caches (32 KB, then 128 KB) each time, at up to ten cycles an instruction, so the set-up
 // keeps one path for every move type and its rare parts out of line.
 #include <cstring>
@@ -782,8 +782,8 @@ __device__ __forceinline__ void load_chunk(const BatchSmem& B, int chunk, int nc
 // distances first, then the next U chunks' loads, then their table reads, without a branch in
 // between -- a lane whose candidate is missing or beyond the cut-off reads row 0 of the table (no vdW)
 // at the cut-off and adds zero.  Energy sums of a move, SM cycles (one chain an SM / 256 chains, two on
-// most SMs): one branching candidate a trip and separate tables 12.6k / 17.8k; U = 2 7.7k / 10.9k,
-// U = 3 7.3k / 10.8k with the whole launch 4% faster / 4% slower (larger code), U = 4 slower for both.
+// most SMs): one branching candidate a trip and separate tables 12.6k / 17.8k; U = 2 7.7k / 10.9k (0.3k / 0.4k
+// more since the reciprocal terms keep their roundings), U = 3 7.3k / 10.8k with the whole launch 4% faster / 4% slower (larger code), U = 4 slower for both.
 template <int KIND, int NT, int U>
 __device__ __forceinline__ void real_space(const BatchSmem& B, double& v1, double& v2) {
   const MoveSmem& M = B.M;

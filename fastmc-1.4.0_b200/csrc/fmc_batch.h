@@ -88,8 +88,10 @@ struct ChainDev {
   double* gasmol;                   // first production samples of N and E per species
   double* gaseng;                   // ([nspecies * 500000 + 1]; null: not recorded)
   long long moves_done;
-  // SM clock cycles spent per phase when the launch is profiled: begin (thread 0), phase
-  // tables, k-space + real space + reduction, end (thread 0), commit
+  // SM clock cycles when the launch is profiled, as thread 0 sees them: [0] set-up, [2] energy sums to the
+  // barrier behind them, [3] acceptance, [4] commit; within the set-up [7] selection and [8] trial and work
+  // list, within the sums [6] warp 0's own; the others stay zero.  A profiled
+  // launch is another build, whose set-up takes some 3k cycles a move longer
   long long prof[12];
   // buffers
   double2* sk;

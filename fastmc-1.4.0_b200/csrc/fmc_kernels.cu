@@ -756,7 +756,8 @@ __device__ __forceinline__ void voxel_centre(const CellGeom& c, int v, int n0, i
 }
 
 // A warp builds the lists of two consecutive voxels (one where a distance takes up to 27 images), 32 atoms
-// at a time: no barriers, and an atom is read once for all of them.  In orthorhombic cells (imcon 1, 2) a distance is taken in float first, which decides all but the atoms within `margin` of the limit; those few
+// at a time: no barriers, and an atom is read once for all of them.  In orthorhombic cells (imcon 1, 2) a
+// distance is taken in float first, which decides all but the atoms within `margin` of the limit; those few
 // are measured in double, so that the lists hold exactly the atoms of the double test.  The margin, with h
 // the longest period and s the largest |atom| + |centre| + h of an axis: rounding the coordinates, their
 // difference and n periods moves a separation by at most 3 * 2^-24 s and its square by h times that; where

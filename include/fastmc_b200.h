@@ -162,7 +162,9 @@ int fmc_ewald1(fmc_chain* c, double* engcpe, int* newld);
 /* ewald1_guest (ewald.f:32-365) for one pass of species `iguest` (0-based) with `natms`
  * sites at xyz.  move: FMC_INSERT, FMC_DELETE, FMC_DISPLACE; pass 1 or 2 for FMC_DISPLACE as
  * in the reference (pass 1 stores the old sites and returns 0; pass 2 returns the energy of
- * the displacement).  S_new stays on the device until fmc_commit. */
+ * the displacement).  S_new stays on the device until fmc_commit.
+ * This call and fmc_guest_realspace return once their energies have arrived: a device failure in what is
+ * left of their kernel, or of an update that fmc_commit left for it to write, is reported by the next call. */
 int fmc_ewald1_guest(fmc_chain* c, int iguest, int natms, const double* xyz, int move, int pass, double* engcpe);
 
 /* guestlistgen + images + ewald2 + srfrce (utility_pack.f:3113-3177, ewald.f:632-694,
