@@ -783,7 +783,8 @@ __device__ __forceinline__ void load_chunk(const BatchSmem& B, int chunk, int nc
 // between -- a lane whose candidate is missing or beyond the cut-off reads row 0 of the table (no vdW)
 // at the cut-off and adds zero.  Energy sums of a move, SM cycles (one chain an SM / 256 chains, two on
 // most SMs): one branching candidate a trip and separate tables 12.6k / 17.8k; U = 2 7.7k / 10.9k (0.3k / 0.4k
-// more since the reciprocal terms keep their roundings), U = 3 7.3k / 10.8k with the whole launch 4% faster / 4% slower (larger code), U = 4 slower for both.
+// more since the reciprocal terms keep their roundings), U = 3 7.3k / 10.8k with the whole launch 4% faster / 4%
+// slower (larger code), U = 4 slower for both.
 template <int KIND, int NT, int U>
 __device__ __forceinline__ void real_space(const BatchSmem& B, double& v1, double& v2) {
   const MoveSmem& M = B.M;
