@@ -669,8 +669,14 @@ void recip_octets(const int* kpacked, int K, std::vector<KOctet>& out) {
 }
 
 double recip_energy_from_parts(const DevSystem& S, const double* host_parts) {
+  // 256 k-vectors at a time, whose sums are then added: the order that energies have always had
   double r = 0.0;
-  for (int b = 0; b < recip_nparts(S); b++) r += host_parts[b];
+  const int n = recip_nparts(S);
+  for (int b = 0; b < n;) {
+    double s = 0.0;
+    for (const int end = std::min(b + 256 / kRecipReduce, n); b < end; b++) s += host_parts[b];
+    r += s;
+  }
   return S.recip_pref * r;
 }
 

@@ -1,10 +1,10 @@
-"""Real-space energies of the plain pass (ewald2 + srfrce), bit for bit.
+"""Real-space energies of the plain pass (ewald2 + srfrce) and the sums over all atoms, bit for bit.
 
 A host move loop over the drop-in calls decides a move that leaves its molecule in place (an angle drawn as exactly
 zero) by what these sums round off: E_new < E_old takes no draw (gcmc.f:1330-1338).  So a seeded loop repeats only
 if every energy keeps its bits.  The oracle rounds differently; the values are those recorded in
 golden/dropin_bits.json with the library of commit f22ff4d: energies of molecules in place, displaced and inserted,
-with and without an update left pending by a commit, and every energy of a plain run.
+with and without an update left pending by a commit, every energy of a plain run, ewald1 and single_point.
 `python tests/test_gpu_dropin_bits.py OUT` records them with the library found on PYTHONPATH."""
 import hashlib
 import json
@@ -35,6 +35,8 @@ CASES = {
     "tilted_slab": ("tilted", 0, ["CO2"], 10, 200),
     "rvdw": ("rvdw", 300, ["CO2"], 20, 200),
     "rvdw_ch4": ("rvdw", 300, ["CH4"], 20, 200),
+    "many_k": ("ortho", 1500, ["CO2"], 60, 100),
+    "many_k_triclinic": ("triclinic", 200, ["CO2", "N2"], 60, 100),
 }
 
 
@@ -52,6 +54,8 @@ def deck(synth, root, name):
         fw = synth.make_framework((28.0,) * 3 if cell == "cubic" else BOX, natoms, seed=natoms)
         if cell == "triclinic":
             fw.cell = fw.cell + np.array([[0, 0, 0], [0.15 * BOX[0], 0, 0], [0, 0.15 * BOX[1], 0]])
+    if name.startswith("many_k"):
+        kmax = (12, 12, 13)
     d = synth.write_inputs(os.path.join(str(root), name), fw, gases, [20.0] * len(gases), 298.0, kmax, imcon=imcon)
     if cell == "rvdw":  # tables of two spacings
         path = os.path.join(d, "CONTROL")
@@ -91,9 +95,10 @@ def values(fmc, synth, root, name):
         c.commit(fmc.DELETE, g, 1)
         out += c.guest_realspace(g, mols[0], 0)
         out += c.guest_realspace(g, mols[2] + 1e-9, 1)
-    assert np.all(np.isfinite(out))
+    sums = [c.ewald1(), *c.single_point()]
+    assert np.all(np.isfinite(out + sums))
     t = fmc.Chain(d, seed=(3, 5, 7, 11)).run(moves)
-    return {"calls": [float(v).hex() for v in out],
+    return {"calls": [float(v).hex() for v in out], "sums": [float(v).hex() for v in sums],
             **{k: hashlib.sha256(np.ascontiguousarray(t[k]).tobytes()).hexdigest()[:24]
                for k in ("mtype", "accepted", "ewld1", "ewld2", "vdw", "estep")}}
 
